@@ -2,7 +2,8 @@
 
 ``listed()`` names twelve such jobs, ``draw(rng)`` makes one more of the same ranges, ``prepare`` builds what the
 program has in hand before the call (weights, inputs, buffers, a model and its captured graph), ``run`` is one pass.
-``work`` counts what a pass cannot do without and ``tolerance`` what another correct implementation may differ by.
+``work`` counts what a pass cannot do without, ``tolerance`` what another correct implementation may differ by, and
+``exact`` evaluates a case in 64 bits with plain torch.
 
 Kinds of case:
   linear     cq_qmatmul / cq_qlinear on device tensors: y = x W^T (+ b) with block-quantized W, one row (decode),
@@ -330,3 +331,90 @@ def tolerance(case):
         return {"rel": {"f32": 1.6e-4, "q8_1": 1e-5, "f16": 1.2e-3}[case["act"]]}
     # logits of f16-operand layers 4.8e-3; one token's f32-mode layers 2.5e-4; two layers of a batch 9e-4
     return {"rel": {"prompt": 1.6e-2, "decode": 1e-3, "layers": 4e-3}[kind]}
+
+
+# ---- the same results in 64 bits, without the library ------------------------------------------------------------
+def _exact_weights(g, qtype, n, k):
+    """The values that the blocks of ``_weights`` stand for, and the scales of the blocks where those are of one kind (f64).
+    The element order inside a block changes nothing here: random bytes come in the files' order only."""
+    if qtype not in ("q4_k", "q6_k"):
+        v = (torch.randn(n, k, generator=g, device="cuda") * 0.02).view(-1, 32)
+        inv = lambda d: torch.where(d != 0, 1.0 / d, torch.zeros_like(d))  # noqa: E731
+        if qtype in ("q4_0", "q5_0"):
+            half = 8 if qtype == "q4_0" else 16
+            d = v.gather(1, v.abs().argmax(1, keepdim=True)) / -half
+            q = (v * inv(d) + (half + 0.5)).int().clamp_max(2 * half - 1) - half
+            w = d.half().double() * q
+        elif qtype == "q4_1":
+            lo = v.amin(1, keepdim=True)
+            d = (v.amax(1, keepdim=True) - lo) / 15
+            w = d.half().double() * ((v - lo) * inv(d) + 0.5).int().clamp_max(15) + lo.half().double()
+        else:
+            d = v.abs().amax(1, keepdim=True) / 127
+            u = (v * inv(d)).double()
+            w = d.half().double() * (u.sign() * (u.abs() + 0.5).floor())  # ties away from zero
+        return w.reshape(n, k), d.half().double().view(n, -1)
+    size = abi.K_BLOCK_BYTES[QTYPES[qtype]]
+    raw = torch.randint(0, 256, (n * (k // 256), size), generator=g, device="cuda", dtype=torch.uint8)
+    scale = lambda lo, hi: (torch.rand(raw.shape[0], 1, generator=g, device="cuda") * (hi - lo) + lo).half().double()  # noqa: E731
+    if qtype == "q4_k":
+        d, dmin = scale(1e-4, 2e-4), scale(8e-4, 1.6e-3)
+        s = raw[:, 4:16].int()
+        sc = torch.cat([s[:, 0:4] & 63, (s[:, 8:12] & 15) | (s[:, 0:4] >> 6 << 4)], 1)
+        mn = torch.cat([s[:, 4:8] & 63, (s[:, 8:12] >> 4) | (s[:, 4:8] >> 6 << 4)], 1)
+        qs = raw[:, 16:].int().view(-1, 4, 1, 32)
+        q = torch.cat([qs & 15, qs >> 4], 2).view(-1, 8, 32)  # 32 low nibbles, then the high ones of the same bytes
+        w = (d * sc).unsqueeze(2) * q - (dmin * mn).unsqueeze(2)
+    else:
+        d = scale(1e-5, 2e-5)
+        ql, qh = raw[:, :128].int().view(-1, 2, 2, 32), raw[:, 128:192].int().view(-1, 2, 1, 32)
+        sc = raw[:, 192:208].view(torch.int8).double().repeat_interleave(16, 1)
+        four = [(ql[:, :, j & 1:(j & 1) + 1] >> (4 * (j >> 1)) & 15) | ((qh >> (2 * j) & 3) << 4) for j in range(4)]
+        w = d * sc * (torch.cat(four, 2).reshape(-1, 256) - 32)
+    return w.reshape(n, k), None
+
+
+def _exact_linear(case, x, w, d):
+    """x W^T; in the Q8_1 mode of the activations that the mode defines: whole numbers of d8 = amax / 127, and for 4-bit
+    weights, whose offset meets a block's sum, that sum in f16 beside them: d4 (sumi d8 - 8 s8)."""
+    if case["act"] != "q8_1":
+        return x.double() @ w.T
+    v = x.reshape(-1, 32)
+    d8 = v.abs().amax(1, keepdim=True) / 127
+    u = torch.where(d8 != 0, v / d8, torch.zeros_like(v)).double()
+    held = d8.half().double() * (u.sign() * (u.abs() + 0.5).floor())
+    y = held.view(x.shape) @ w.T
+    if case["qtype"] == "q4_0":
+        y += (held.sum(1) - v.sum(1, dtype=torch.float64).half().double()).view(x.shape[0], -1) @ (8 * d).T
+    return y
+
+
+def exact(case, seed):
+    kind = case["kind"]
+    if kind in ("decode", "prompt", "layers"):  # their weights and caches come from the library's own generator
+        return None
+    g = _generator(seed)
+    if kind in ("linear", "forward"):
+        m, n, k = case["m"], case["n"], case["k"]
+        w, d = _exact_weights(g, case["qtype"], n, k)
+        if kind == "forward":
+            x = torch.from_numpy(np.random.default_rng(int(seed)).standard_normal((m, k), dtype=np.float32)).cuda()
+            return _exact_linear(case, x, w, d).cpu().numpy()
+        y = _exact_linear(case, torch.randn(m, k, generator=g, device="cuda"), w, d)
+        return y + (torch.randn(n, generator=g, device="cuda") * 0.1).double() if case["bias"] else y
+    if kind == "codec":  # the blocks are bytes
+        return None, _exact_weights(g, case["qtype"], case["n"], case["k"])[0]
+    b, h, hk, sq, sk, dim = (case[x] for x in ("b", "h", "hk", "sq", "sk", "d"))
+    dt = torch.bfloat16 if case["bf16"] else torch.float16
+    q, key, v = (torch.randn(b, s, heads, dim, generator=g, device="cuda").to(dt) for s, heads in ((sq, h), (sk, hk), (sk, hk)))
+    hidden = torch.ones(sq, sk, dtype=torch.bool, device="cuda").triu(1 + sk - sq) if case["causal"] else None
+    o = torch.empty(b, sq, h, dim, dtype=torch.float64, device="cuda")
+    lse = torch.empty(b, h, sq, dtype=torch.float64, device="cuda")
+    for i in range(b):
+        for j in range(h):
+            s = q[i, :, j].double() @ key[i, :, j * hk // h].double().T * dim ** -0.5
+            if hidden is not None:
+                s.masked_fill_(hidden, -math.inf)
+            lse[i, j] = s.logsumexp(1)
+            o[i, :, j] = (s - lse[i, j].unsqueeze(1)).exp_() @ v[i, :, j * hk // h].double()
+    return o, lse

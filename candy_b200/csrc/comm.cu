@@ -151,7 +151,7 @@ cq_status cq_comm_create(cq_ctx *ctx, int rank, int world, int64_t max_floats, c
     cq_comm *c = new cq_comm();
     c->rank = rank, c->world = world, c->max_floats = (size_t)max_floats;
     const size_t bytes = comm_bytes(world, c->max_floats);
-    cudaError_t e = cudaMalloc(&c->local, bytes);
+    cudaError_t e = cq_device_malloc(ctx, (void **)&c->local, bytes);
     if (e == cudaSuccess) e = cudaMemset(c->local, 0, bytes);
     if (e == cudaSuccess) e = cudaIpcGetMemHandle(reinterpret_cast<cudaIpcMemHandle_t *>(handle64), c->local);
     if (e != cudaSuccess) {
@@ -181,7 +181,7 @@ cq_status cq_comm_connect(cq_ctx *ctx, cq_comm *c, const void *all_handles) {
     for (int set = 0; set < 2; ++set) {
         std::vector<uint2 *> rx(c->world);
         for (int r = 0; r < c->world; ++r) rx[r] = slot_ptr(c->peer_base[r], c->world, c->max_floats, set, c->rank);
-        CQ_CUDA(ctx, cudaMalloc((void **)&c->d_push_rx[set], sizeof(uint2 *) * c->world));
+        CQ_CUDA(ctx, cq_device_malloc(ctx, (void **)&c->d_push_rx[set], sizeof(uint2 *) * c->world));
         CQ_CUDA(ctx, cudaMemcpy(c->d_push_rx[set], rx.data(), sizeof(uint2 *) * c->world, cudaMemcpyHostToDevice));
     }
     return CQ_OK;

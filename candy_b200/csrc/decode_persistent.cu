@@ -637,7 +637,7 @@ bool ps_plan_linear(PsOp &op, int n, int k, int block_bytes, bool even_rows) {
 template <typename T>
 cq_status ps_alloc(cq_ctx *ctx, cq_decoder *dec, T **out, size_t count, bool zero) {
     void *ptr = nullptr;
-    CQ_CUDA(ctx, cudaMalloc(&ptr, count * sizeof(T)));
+    CQ_CUDA(ctx, cq_device_malloc(ctx, &ptr, count * sizeof(T)));
     dec->owned.push_back(ptr);
     if (zero) CQ_CUDA(ctx, cudaMemsetAsync(ptr, 0, count * sizeof(T), ctx->stream));
     *out = static_cast<T *>(ptr);
@@ -768,7 +768,7 @@ cq_status cq_decoder_create(cq_ctx *ctx, const cq_decoder_desc *desc, cq_decoder
     p.stash_off = (int)(stages * stage_bytes), p.coop_off = p.stash_off + (int)stash_bytes, p.xs_off = p.coop_off + (int)coop_bytes;
     dec->smem = (size_t)p.xs_off + xs_bytes;
     dec->grid = ctx->sm_count;
-    CQ_CUDA(ctx, cudaMalloc((void **)&dec->ops_dev, dec->ops.size() * sizeof(PsOp)));
+    CQ_CUDA(ctx, cq_device_malloc(ctx, (void **)&dec->ops_dev, dec->ops.size() * sizeof(PsOp)));
     dec->owned.push_back(dec->ops_dev);
     CQ_CUDA(ctx, cudaMemcpyAsync(dec->ops_dev, dec->ops.data(), dec->ops.size() * sizeof(PsOp), cudaMemcpyHostToDevice, ctx->stream));
     CQ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

@@ -884,7 +884,7 @@ cq_status launch_gemm(cq_ctx *ctx, int qtype, int order, int actmode, const floa
             if (ctx->capturing || (cudaStreamIsCapturing(ctx->stream, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone))
                 return cq_fail(ctx, CQ_ERR_INVALID_ARG, "gemm: the cached f16 copy of this weight matrix does not exist yet and cannot be allocated during stream capture: run the call once before capturing");
             void *p = nullptr;
-            CQ_CUDA(ctx, cudaMalloc(&p, w16_bytes));
+            CQ_CUDA(ctx, cq_device_malloc(ctx, &p, w16_bytes));
             ctx->w16_cache[key] = p;
             ctx->w16_cache_bytes += w16_bytes;
             w16 = static_cast<__half *>(p);

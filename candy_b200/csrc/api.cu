@@ -212,6 +212,7 @@ cq_status cq_ctx_set_option(cq_ctx *ctx, const char *key, int64_t value) {
     else if (!strcmp(key, "comm_poll_limit")) t.comm_poll_limit = (int)value;
     else if (!strcmp(key, "comm_cluster")) t.comm_cluster = (int)value;
     else if (!strcmp(key, "gemm_int8")) t.gemm_int8 = (int)value;
+    else if (!strcmp(key, "split_min_rows")) t.split_min_rows = (int)value;
     else if (!strcmp(key, "i8_min_rows_f32")) t.i8_min_rows_f32 = (int)value;
     else if (!strcmp(key, "i8_min_rows_q8_1")) t.i8_min_rows_q8_1 = (int)value;
     else if (!strcmp(key, "gemv_mma")) t.gemv_mma = (int)value;
@@ -428,6 +429,14 @@ cq_status cq_qmatmul(cq_ctx *ctx, int qtype, int order, int actmode, const float
         if (s == CQ_OK && ctx->bias) ctx->bias_done = true;
         return s;
     }
+    // CQ_ACT_F32 from nine rows on: both operands as sums of two f16 numbers on CTA pairs (n 11008, k 4096, us, the integer
+    // kernel's planes in brackets: 9 rows 21 (28), 128 rows 43 (104), 512 rows 109 (409); up to eight rows the streaming kernel
+    // takes 12.7, or for Q8_0 the planes 18.9 against 21).  Only where the planes served before: an x without 16-byte
+    // alignment keeps its plain f32 arithmetic.
+    if (actmode == CQ_ACT_F32 && ctx->tune.split_min_rows > 0 && m >= ctx->tune.split_min_rows && ctx->tune.gemm_int8 && !ctx->fuse.on && ctx->push.world == 0 &&
+        ctx->tune.gemv_variant == 0 && !ctx->tune.force_simple && gemm_pair_tmem_supported(qtype, k, w_blocks_dev) &&
+        qgemm_i8_supported(qtype, k, w_blocks_dev, x_dev, ldx))
+        return launch_gemm_pair_tmem(ctx, qtype, order, true, x_dev, m, k, ldx, w_blocks_dev, n, y_dev, ldy);
     // Integer dots on the tensor cores: one weight pass for the whole batch, in the activation mode's own numerics.
     if (actmode != CQ_ACT_F16 && ctx->tune.gemm_int8 && !ctx->fuse.on && ctx->push.world == 0 && ctx->tune.gemv_variant == 0 &&
         m >= (actmode == CQ_ACT_Q8_1 ? ctx->tune.i8_min_rows_q8_1 : ctx->tune.i8_min_rows_f32) &&

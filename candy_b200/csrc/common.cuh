@@ -47,7 +47,8 @@ struct GemvTuning {
     int gemm_int8 = 1;        // 1: the int8 tensor-core kernel serves CQ_ACT_Q8_1 from i8_min_rows_q8_1 rows and CQ_ACT_F32 from i8_min_rows_f32 rows
     int64_t host_zero_copy = 256 << 10;  // cq_qmatmul_host, m <= 8: a result of up to this many bytes whose buffer is pinned host memory is written in place (0: always copy out)
     int gemm_pair = 1;           // m > 128: 256 x 256 tiles on CTA pairs (cta_group::2) instead of 128 x 256 per CTA
-    int gemm_fused_dequant = 1;  // Q4_0, m > 128: dequantize inside the f16 GEMM's producer instead of making an f16 copy of W (1: up to 384 rows, 2: always)
+    int gemm_fused_dequant = 1;  // CQ_ACT_F16, Q4_0 / Q8_0: the CTA-pair kernel that dequantizes in place (1: where it is the quicker one, 2: every batch of nine and more, 0: never)
+    int split_min_rows = 9;      // CQ_ACT_F32 batches of this many rows: both operands as sums of two f16 numbers (0: never)
     int i8_min_rows_f32 = 3;
     int i8_min_rows_q8_1 = 3;
     int gemv_mma = 3;       // CQ_ACT_F32, Q4_0: batches of this many rows up to 8 take the single-launch mma.sync kernel (0: never)
@@ -178,6 +179,11 @@ cq_status launch_gemv_mma_f16(cq_ctx *ctx, int order, const float *x, int64_t m,
                               float *y, int64_t ldy);
 cq_status launch_qgemm_i8(cq_ctx *ctx, int qtype, int order, int mode, const float *x, int64_t m, int64_t k, int64_t ldx, const void *w, int64_t n,
                           float *y, int64_t ldy);
+// Batches on CTA pairs, raw blocks dequantized into tensor memory (gemm_pair_tmem.cu): split = CQ_ACT_F32 by sums of two
+// f16 numbers, otherwise CQ_ACT_F16.
+bool gemm_pair_tmem_supported(int qtype, int64_t k, const void *w);
+cq_status launch_gemm_pair_tmem(cq_ctx *ctx, int qtype, int order, bool split, const float *x, int64_t m, int64_t k, int64_t ldx, const void *w, int64_t n,
+                                float *y, int64_t ldy);
 cq_status launch_gemm(cq_ctx *ctx, int qtype, int order, int actmode, const float *x, int64_t m, int64_t k,
                       int64_t ldx, const void *w, int64_t n, float *y, int64_t ldy);
 

@@ -112,12 +112,14 @@ cq_status cq_ctx_set_option(cq_ctx *ctx, const char *key, int64_t value);
  * single-launch kernel with mma.sync block dots, two rows too against large weights, and CQ_ACT_F16 batches of up to
  * eight rows its f16 form; 0: never); gemv_force_simple; gemm_variant, gemm_cache_weights (keep an f16 copy of each weight matrix the wide
  * GEMM has seen: the weights must then stay unchanged, or be rewritten only through cq_* entry points, or
- * cq_invalidate_weight_cache must be called); gemm_pair (1, default: CQ_ACT_F16 batches beyond 384 rows run 256 x 256
- * tiles on CTA pairs; 0: 128 x 256 tiles per CTA); gemm_fused_dequant (1, default: Q4_0 batches of 129..384 rows in
- * CQ_ACT_F16 dequantize the raw blocks inside the GEMM instead of making an f16 copy of W; 2: at every batch size;
- * 0: never); gemm_int8 (1, default: batches of i8_min_rows_q8_1 (3) or more
- * rows in CQ_ACT_Q8_1 and of i8_min_rows_f32 (3) or more in CQ_ACT_F32 run the int8 tensor-core kernel, one
- * weight pass per batch; 0: the decode kernels, up to eight rows a pass); attn_variant (decode attention: 1 = one CTA per 32-key chunk for grouped heads instead of split contexts, 2 = never the
+ * cq_invalidate_weight_cache must be called); gemm_pair (1, default: CQ_ACT_F16 batches that work from an f16 copy
+ * of W run 256 x 256 tiles on CTA pairs; 0: 128 x 256 tiles per CTA); gemm_fused_dequant (1, default: Q4_0 and Q8_0
+ * batches of up to 1024 rows in CQ_ACT_F16 dequantize the raw blocks inside a CTA-pair GEMM where that is quicker than
+ * the other routes; 2: at every batch size; 0: never); gemm_int8 (1, default: batches of i8_min_rows_q8_1 (3) or more
+ * rows in CQ_ACT_Q8_1 and of i8_min_rows_f32 (3) or more in CQ_ACT_F32 run on the tensor cores, one
+ * weight pass per batch; 0: the decode kernels, up to eight rows a pass); split_min_rows (9, default: CQ_ACT_F32
+ * batches of this many rows multiply sums of two f16 numbers, in effect 22-bit operands; 0: the int8 kernel serves
+ * them too); attn_variant (decode attention: 1 = one CTA per 32-key chunk for grouped heads instead of split contexts, 2 = never the
  * single-launch cluster kernel of short contexts); comm_poll_limit (polls before the reducing
  * norm gives up on a peer's data, default about one second's worth); comm_cluster; host_zero_copy (see
  * cq_qmatmul_host); fa_transpose_v (1: cq_flash_attention always transposes V into scratch first; 0, default: V tiles
@@ -179,9 +181,10 @@ cq_status cq_quantize_q8_1(cq_ctx *ctx, const float *x_dev, int64_t m, int64_t k
  * (quantized.cu:1323), mul_mat_vec_q4_0_q8_1_cuda1..8 (quantized.cu:2874-3519) and
  * mul_mat_q4_0 / mul_mat_q8_0 (quantized.cu:4477, :4529).
  * One row runs the streaming decode GEMV; batches in CQ_ACT_F32 / CQ_ACT_Q8_1 run integer dots per quant block on
- * the tensor cores, scaled per block as the mode says (CQ_ACT_F32 batches hold each activation block as 15-bit
- * block fixed point, about 2e-5 of max|y| from the CPU path; CQ_ACT_Q8_1 batches quantize exactly as quantize_q8_1
- * does; up to eight rows against Q4_0 run in a single-launch streaming kernel, larger batches in the int8 GEMM);
+ * the tensor cores, scaled per block as the mode says (CQ_ACT_F32 batches of up to eight rows hold each activation
+ * block as 15-bit block fixed point, about 2e-5 of max|y| from the CPU path, larger ones multiply sums of two f16
+ * numbers, within 1e-5; CQ_ACT_Q8_1 batches quantize exactly as quantize_q8_1 does; up to eight rows against Q4_0 run
+ * in a single-launch streaming kernel, larger Q8_1 batches in the int8 GEMM);
  * CQ_ACT_F16 runs the f16 tensor-core GEMMs (up to eight rows against Q4_0: the single-launch streaming kernel with
  * f16 operands, same rounding of the operands).
  * Preconditions: k % 32 == 0, k >= 32, m, n >= 1, ldx >= k, ldy >= n. */

@@ -1,0 +1,109 @@
+"""The CTA-pair GEMM (raw blocks dequantized into tensor memory): CQ_ACT_F32 as sums of two f16 numbers, and CQ_ACT_F16,
+at the edges of its tiles (256 weight rows, 32 / 64 / 128 batch rows, chunks of 256 k, shares that cut a tile) against f64."""
+import numpy as np
+import pytest
+
+from candy_b200 import abi
+from candy_b200.backend import ACT_F16, ACT_F32, QStorage
+from oracle import oracle_c as oc
+
+pytestmark = pytest.mark.gpu
+
+
+def tol(k):
+    """The tensor core truncates when it adds: up to 2^-23 of the sum per K = 16 step; 2^-20 for the operands' last bits."""
+    return k / 16 * 2.0 ** -23 + 2.0 ** -20
+
+
+def call(device, qt, order, x, ldx, blocks, n, act, bias=None, ldy=None):
+    m, k = x.shape
+    ldy = ldy or n
+    xs = np.full((m, ldx), 7.0, dtype=np.float32)
+    xs[:, :k] = x
+    qs = QStorage.from_blocks(device, qt, order, n, k, blocks)
+    xd, yd = device.storage_from_slice(xs), device.storage_from_slice(np.full((m, ldy), -77.0, dtype=np.float32))
+    bd = device.storage_from_slice(bias) if bias is not None else None
+    st = device._lib.cq_qlinear(device.ctx, qt, order, act, xd.ptr, m, k, ldx, qs.buf.ptr, n, bd.ptr if bd else None, yd.ptr, ldy)
+    abi.check(device.ctx, st, "linear")
+    device.synchronize()
+    y = yd.data().reshape(m, ldy)
+    assert (y[:, n:] == -77.0).all()
+    return y[:, :n]
+
+
+def err(y, want):
+    return float(np.abs(y - want).max() / np.abs(want).max())
+
+
+@pytest.mark.parametrize("qt,order", [(oc.Q4_0, 0), (oc.Q4_0, 1), (oc.Q8_0, 0)])
+@pytest.mark.parametrize("m,n,k", [(9, 1, 256), (16, 127, 512), (32, 256, 256), (33, 257, 768), (64, 700, 2304), (65, 129, 256), (100, 1000, 4096),
+                                   (128, 5000, 1024), (129, 300, 512), (300, 2000, 768)])
+def test_split_f32(device, qt, order, m, n, k):
+    rng = np.random.default_rng(m + n + k + order)
+    blocks = oc.quantize(qt, order, (rng.standard_normal((n, k)) * 0.02).astype(np.float32))
+    x = (rng.standard_normal((m, k)) * 10.0 ** rng.uniform(-6, 6, (m, 1))).astype(np.float32)  # rows of very different size
+    x[m // 2] = 0.0
+    bias = rng.standard_normal(n).astype(np.float32) if n > 200 else None
+    y = call(device, qt, order, x, k + 4, blocks, n, ACT_F32, bias, n + 3)
+    w = oc.dequantize(qt, order, blocks.reshape(-1)).reshape(n, k).astype(np.float64)
+    want = x.astype(np.float64) @ w.T
+    if bias is not None:
+        y, want = y - np.zeros((1, n), np.float32), want + bias
+    for r in range(m):  # row by row: each has its own scale
+        top = np.abs(want[r]).max()
+        assert np.abs(y[r] - want[r]).max() <= tol(k) * max(np.abs(x[r].astype(np.float64) @ w.T).max(), 0.0) * 4 + 2.0 ** -23 * top
+
+
+@pytest.mark.parametrize("qt,limit", [(oc.Q4_0, 0x6C00), (oc.Q8_0, 0x6000)])
+def test_split_with_scales_near_f16s_limits(device, qt, limit):
+    """Scales whose products leave f16's range (those rows are computed in f32), the largest that do not, and subnormal ones."""
+    n, k, m = 300, 512, 20
+    rng = np.random.default_rng(3)
+    blocks = rng.integers(0, 256, size=(n, k // 32, abi.BLOCK_BYTES[qt]), dtype=np.uint8)
+    rows = {0: limit - 1, 5: limit, 131: 0x7BFF, 200: 0x0001, 201: 0x03FF, 299: 0xFBFF}
+    d = np.full((n, k // 32), 0x2000, dtype=np.uint16)
+    for r, bits in rows.items():
+        d[r, rng.integers(0, k // 32)] = bits
+        if bits < 0x0400:
+            d[r] = bits
+    blocks[:, :, 0], blocks[:, :, 1] = d & 0xFF, d >> 8
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    y = call(device, qt, 0, x, k, blocks.reshape(-1), n, ACT_F32)
+    w = oc.dequantize(qt, 0, blocks.reshape(-1)).reshape(n, k).astype(np.float64)
+    want = x.astype(np.float64) @ w.T
+    for j in range(n):
+        assert np.abs(y[:, j] - want[:, j]).max() <= 4 * tol(k) * np.abs(want[:, j]).max()
+
+
+def test_split_keeps_nan_and_inf_in_their_rows(device):
+    n, k, m = 256, 256, 40
+    rng = np.random.default_rng(4)
+    blocks = oc.quantize(oc.Q4_0, 0, rng.standard_normal((n, k)).astype(np.float32))
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    clean = call(device, oc.Q4_0, 0, x, k, blocks, n, ACT_F32)
+    x[3, 7], x[39, 255] = np.nan, np.inf
+    y = call(device, oc.Q4_0, 0, x, k, blocks, n, ACT_F32)
+    keep = [r for r in range(m) if r not in (3, 39)]
+    assert (y[keep] == clean[keep]).all()
+    assert not np.isfinite(y[3]).any() and not np.isfinite(y[39]).any()
+
+
+@pytest.mark.parametrize("qt", [oc.Q4_0, oc.Q8_0])
+@pytest.mark.parametrize("m,n,k", [(1, 300, 256), (31, 256, 512), (64, 129, 2304), (70, 3000, 1024), (128, 257, 256), (200, 700, 768)])
+def test_f16_on_pairs(device, qt, m, n, k):
+    rng = np.random.default_rng(m + n + k)
+    blocks = oc.quantize(qt, 0, (rng.standard_normal((n, k)) * 0.02).astype(np.float32))
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    bias = rng.standard_normal(n).astype(np.float32)
+    device.set_option("gemm_fused_dequant", 2)
+    device.set_option("gemv_mma", 0)
+    try:
+        y = call(device, qt, 0, x, k, blocks, n, ACT_F16, bias)
+        again = call(device, qt, 0, x, k, blocks, n, ACT_F16, bias)
+    finally:
+        device.set_option("gemm_fused_dequant", 1)
+        device.set_option("gemv_mma", 3)
+    w16 = oc.dequantize(qt, 0, blocks.reshape(-1)).reshape(n, k).astype(np.float16).astype(np.float64)
+    want = x.astype(np.float16).astype(np.float64) @ w16.T + bias
+    assert err(y, want) < tol(k) * 4
+    assert (y == again).all()  # partial tiles are added in a fixed order

@@ -17,7 +17,9 @@
 //   warp 10       tcgen05.mma issue of O_tile = P V, with P read from tensor memory as the A operand, into one of two
 //                 product slots; one commit per product.  Two issuing threads because one thread issues an
 //                 M 128 x N 128 x K 16 instruction every ~100 cycles while the tensor pipe needs 64: with both products on
-//                 one thread the issue was the longest role of a tile (2 x 64/8 heads x 4096: 732 -> 659 us)
+//                 one thread the issue was the longest role of a tile (2 x 64/8 heads x 4096: 732 -> 659 us).  All lanes
+//                 of a warp run its issuing loop and one issues, so that descriptors stay in uniform registers
+//                 (2 x 64/8 heads x 4096: 708 -> 684 us)
 //   warps 2-9     compute: thread = (query row, half of the columns): warps 2-5 take keys 0-63 of a tile and the first
 //                 half of the output row, warps 6-9 the other halves (two warps per tensor-memory lane quarter, two per
 //                 scheduler).  Softmax of the half: scores read once (tcgen05.ld, loads in flight together), masked
@@ -154,7 +156,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
              *o_full = p_full + 2, *o_empty = o_full + 2;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(o_empty + 2);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     // A CTA stays on its SM and takes one work item per round: an item is one tile of 128 query rows of one (head, batch).
     // Items are numbered heavy first (late query rows under a causal mask have the most key tiles) and dealt out in
     // alternating directions, which gives every CTA a similar load.  Between items nothing is torn down: the next
@@ -287,7 +289,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
         // ---- first MMA issuer: S(t) = Q K(t)^T, as far ahead as the K ring and the score slot allow ----------------------
         // (one thread issues an M 128 x N 128 x K 16 instruction every ~100 cycles, the tensor pipe needs 64: with the two
         // products on one thread the issue was the tile's longest role, with a thread each they run side by side)
-        if (lane == 0) {
+        {  // the whole warp runs the loop, one lane issues
             constexpr uint32_t idesc_s = idesc_16(FA_M, FA_N, BF16);
             const uint32_t q_addr = smem_u32(sm_q);
             bool ok = true;
@@ -298,7 +300,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
                 int q0, head, batch, ntiles;
                 item_at(w, q0, head, batch, ntiles);
                 if (ntiles == 0) continue;
-                if (!mbar_wait_bounded(smem_u32(q_full), qi & 1)) {
+                if (!__all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(q_full), qi & 1))) {
                     ok = false;
                     break;
                 }
@@ -306,30 +308,34 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
                     const int gt = g + t, s = gt % KS;
                     // the K tile has landed; the score slot is free (one slot: the softmax warps free it as soon as they hold
                     // the previous tile's scores in registers)
-                    if (!mbar_wait_bounded(smem_u32(&k_full[s]), (gt / KS) & 1) || (gt >= 1 && !mbar_wait_bounded(smem_u32(s_empty), (gt - 1) & 1))) {
+                    const bool there = mbar_wait_bounded(smem_u32(&k_full[s]), (gt / KS) & 1) && (gt < 1 || mbar_wait_bounded(smem_u32(s_empty), (gt - 1) & 1));
+                    if (!__all_sync(0xffffffffu, there)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
                     const uint32_t k_addr = smem_u32(sm_k + (size_t)s * Cfg::kKBytes);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int c = 0; c < SLABS; ++c)
+                        for (int c = 0; c < SLABS; ++c)
 #pragma unroll
-                        for (int kk = 0; kk < 4; ++kk)
-                            tc_mma_f16(tmem_base + Cfg::kColS, smem_desc_k128(q_addr + c * (FA_M * 128) + kk * 32),
-                                       smem_desc_k128(k_addr + c * (FA_N * 128) + kk * 32), idesc_s, (c | kk) != 0);
-                    tc_commit(smem_u32(s_full));
-                    tc_commit(smem_u32(&k_empty[s]));  // the K tile is free once these MMAs have read it
-                    if (t == ntiles - 1) tc_commit(smem_u32(q_empty));  // and so is Q after the item's last score tile
+                            for (int kk = 0; kk < 4; ++kk)
+                                tc_mma_f16(tmem_base + Cfg::kColS, smem_desc_k128(q_addr + c * (FA_M * 128) + kk * 32),
+                                           smem_desc_k128(k_addr + c * (FA_N * 128) + kk * 32), idesc_s, (c | kk) != 0);
+                        tc_commit(smem_u32(s_full));
+                        tc_commit(smem_u32(&k_empty[s]));  // the K tile is free once these MMAs have read it
+                        if (t == ntiles - 1) tc_commit(smem_u32(q_empty));  // and so is Q after the item's last score tile
+                    }
+                    __syncwarp();
                 }
                 g += ntiles;
                 ++qi;
             }
-            if (!ok) atomicExch(p.err, kDevErrMma);
+            if (!ok && lane == 0) atomicExch(p.err, kDevErrMma);
         }
     } else if (warp == FA_THREADS / 32 - 1) {
         // ---- second MMA issuer: O_tile(t) = P(t) V(t), P from tensor memory as the A operand ----------------------------
-        if (lane == 0) {
+        {
             constexpr uint32_t idesc_o = idesc_16(FA_M, D, BF16);
             bool ok = true;
             int g = 0;
@@ -341,28 +347,32 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
                 for (int j = 0; j < ntiles && ok; ++j) {
                     const int gj = g + j, s = gj % VS, slot = gj & 1;
                     // V and P in place, and the product slot free (the compute warps have folded the tile two back)
-                    if (!mbar_wait_bounded(smem_u32(&v_full[s]), (gj / VS) & 1) || !mbar_wait_bounded(smem_u32(&p_full[slot]), (gj >> 1) & 1) ||
-                        (gj >= 2 && !mbar_wait_bounded(smem_u32(&o_empty[slot]), ((gj >> 1) - 1) & 1))) {
+                    const bool there = mbar_wait_bounded(smem_u32(&v_full[s]), (gj / VS) & 1) && mbar_wait_bounded(smem_u32(&p_full[slot]), (gj >> 1) & 1) &&
+                                       (gj < 2 || mbar_wait_bounded(smem_u32(&o_empty[slot]), ((gj >> 1) - 1) & 1));
+                    if (!__all_sync(0xffffffffu, there)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
                     const uint32_t v_addr = smem_u32(sm_v + (size_t)s * Cfg::kVBytes);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int hf = 0; hf < 2; ++hf)
+                        for (int hf = 0; hf < 2; ++hf)
 #pragma unroll
-                        for (int kk = 0; kk < 4; ++kk) {  // 16 keys per step: 8 tensor-memory columns of P
-                            // V^T: 32 bytes further along a row of 64 keys (K-major operand).  V itself: 16 rows of 128 bytes further
-                            // down (the operand is N-major: d runs along a row, 64-wide slabs of d lie FA_N * 128 bytes apart)
-                            const uint64_t bdesc = VT ? smem_desc_k128(v_addr + hf * (D * 128) + kk * 32) : smem_desc_mn128(v_addr + (hf * 4 + kk) * 2048, FA_N * 128);
-                            tc_mma_f16_ts(tmem_base + Cfg::kColO + (uint32_t)(slot * D), tmem_base + Cfg::kColP + (uint32_t)(slot * 64 + (hf * 4 + kk) * 8), bdesc,
-                                          VT ? idesc_o : (idesc_o | (1u << 16)), (hf | kk) != 0);
-                        }
-                    tc_commit(smem_u32(&o_full[slot]));  // product ready; its P slot and V stage free
+                            for (int kk = 0; kk < 4; ++kk) {  // 16 keys per step: 8 tensor-memory columns of P
+                                // V^T: 32 bytes further along a row of 64 keys (K-major operand).  V itself: 16 rows of 128 bytes further
+                                // down (the operand is N-major: d runs along a row, 64-wide slabs of d lie FA_N * 128 bytes apart)
+                                const uint64_t bdesc = VT ? smem_desc_k128(v_addr + hf * (D * 128) + kk * 32) : smem_desc_mn128(v_addr + (hf * 4 + kk) * 2048, FA_N * 128);
+                                tc_mma_f16_ts(tmem_base + Cfg::kColO + (uint32_t)(slot * D), tmem_base + Cfg::kColP + (uint32_t)(slot * 64 + (hf * 4 + kk) * 8), bdesc,
+                                              VT ? idesc_o : (idesc_o | (1u << 16)), (hf | kk) != 0);
+                            }
+                        tc_commit(smem_u32(&o_full[slot]));  // product ready; its P slot and V stage free
+                    }
+                    __syncwarp();
                 }
                 g += ntiles;
             }
-            if (!ok) atomicExch(p.err, kDevErrMma);
+            if (!ok && lane == 0) atomicExch(p.err, kDevErrMma);
         }
     } else {
         // ---- eight compute warps: thread = (query row, one half of the columns) ------------------------------------------

@@ -36,7 +36,7 @@ constexpr int I8_ROWS = 128;     // weight rows per tile
 constexpr int I8_KCHUNK = 256;   // values of k per item (eight quant blocks)
 constexpr int I8_BLOCKS = 8;
 
-template <int QT, int NC>
+template <int QT, int MODE, int NC>
 struct I8Cfg {
     static constexpr int kBlockBytes = QT == CQ_Q4_0 ? kQ4Bytes : kQ8Bytes;
     static constexpr int kRowChunk = I8_BLOCKS * kBlockBytes;     // raw bytes of one row per item: 144 / 272
@@ -48,7 +48,9 @@ struct I8Cfg {
     static constexpr int kBBytes = NC * I8_KCHUNK;                // activation columns: two [NC x 128 B] halves
     static constexpr int kBStages = NC <= 32 ? 4 : (NC <= 64 ? 3 : 2);  // the epilogue holds a stage (its scales) to the end of the chunk
     static constexpr int kXScaleBytes = I8_BLOCKS * NC * 8;       // float2 per (block, column) (plane mode uses half)
-    static constexpr int kEpWarps = NC >= 128 ? 8 : 4;
+    // wide Q8_1 tiles: sixteen warps of 32 columns, which hide the latency of reading tensor memory among themselves; else four or
+    // eight that fetch ahead
+    static constexpr int kEpWarps = NC >= 128 ? (MODE == 1 ? 16 : 8) : (NC >= 64 && MODE == 1 ? 8 : 4);
     static constexpr int kColsPerWarp = NC / (kEpWarps / 4);
     // Accumulator slots in tensor memory, handed over in two groups: the MMAs of a group are committed once and
     // the epilogue takes a whole group per barrier round (NC <= 32: a group is a chunk's eight blocks).
@@ -115,7 +117,7 @@ __global__ void __launch_bounds__(256) i8_prepass_kernel(const float *__restrict
             q[2] = amax == 0.0f ? 0 : (int)roundf(__fdiv_rn(v.z, d));
             q[3] = amax == 0.0f ? 0 : (int)roundf(__fdiv_rn(v.w, d));
             sc.x = __half2float(__float2half_rn(d));
-            sc.y = __half2float(__float2half_rn(sum));
+            sc.y = -8.0f * __half2float(__float2half_rn(sum));  // (exact) as the Q4_0 epilogue uses it
         } else {
             const float inv = amax > 0.0f ? 16383.0f / amax : 0.0f;
             q[0] = __float2int_rn(fminf(fmaxf(v.x * inv, -16383.0f), 16383.0f));
@@ -146,7 +148,12 @@ __global__ void __launch_bounds__(256) i8_prepass_kernel(const float *__restrict
                 *reinterpret_cast<uint32_t *>(dst + 4 * l) = byte[0] | (byte[1] << 8) | (byte[2] << 16) | (byte[3] << 24);
             }
         }
-        if (l == 0) scale[((int64_t)(row / ncl) * nb + b) * ncl + (row % ncl)] = sc;
+        if (l == 0 && MODE == 0) scale[((int64_t)(row / ncl) * nb + b) * ncl + (row % ncl)] = sc;
+        if (l == 0 && MODE == 1) {  // columns in pairs, (x0, x1, y0, y1): the packed epilogue takes two columns per instruction
+            const int c = row % ncl;
+            float *dst = reinterpret_cast<float *>(scale + ((int64_t)(row / ncl) * nb + b) * ncl + (c & ~1)) + (c & 1);
+            dst[0] = sc.x, dst[2] = sc.y;
+        }
     }
 }
 
@@ -195,9 +202,9 @@ __device__ __forceinline__ void row_words(const uint32_t (&row)[ROWW], int hw, u
 
 // MODE 1: Q8_1 columns, MODE 0: hi / lo plane columns (NC tensor-memory columns = NC / 2 activation rows).
 template <int QT, int MODE, int NC>
-__global__ void __launch_bounds__(I8Cfg<QT, NC>::kThreads, 1)
+__global__ void __launch_bounds__(I8Cfg<QT, MODE, NC>::kThreads, 1)
     qgemm_i8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const I8Params p) {
-    using Cfg = I8Cfg<QT, NC>;
+    using Cfg = I8Cfg<QT, MODE, NC>;
     constexpr int WST = Cfg::kWStages, AST = Cfg::kAStages, BST = Cfg::kBStages, GROUP = Cfg::kGroup, EPW = Cfg::kEpWarps;
     constexpr int NCL = MODE == 1 ? NC : NC / 2;  // logical columns (activation rows) of the launch
     extern __shared__ uint8_t smem_raw[];
@@ -212,7 +219,7 @@ __global__ void __launch_bounds__(I8Cfg<QT, NC>::kThreads, 1)
              *b_empty = b_full + BST, *s_full = b_empty + BST, *s_empty = s_full + 2;  // one pair per group of slots
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(s_empty + 2);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     pdl_launch_dependents();
     const int g0 = blockIdx.x * p.per_cta, g1 = min(g0 + p.per_cta, p.total);
 
@@ -311,40 +318,46 @@ __global__ void __launch_bounds__(I8Cfg<QT, NC>::kThreads, 1)
                     }
         }
     } else if (warp == 2) {
-        // ---- MMA: one K = 32 instruction per quant block, each into its own tensor-memory slot ----------
-        if (lane == 0) {
+        // ---- MMA: one K = 32 instruction per quant block, each into its own tensor-memory slot (the whole warp runs the
+        // loop, one lane issues) ----
+        {
             constexpr uint32_t idesc = idesc_i8(I8_ROWS, NC, QT == CQ_Q8_0);
             int st = 0, gi = 0;  // chunks and groups of blocks issued so far
             bool ok = true;
             for (int g = g0; g < g1 && ok; ++g, ++st) {
                 const int sa = st % AST, sb = st % BST;
-                if (!mbar_wait_sleep(smem_u32(&a_full[sa]), (st / AST) & 1, 40) || !mbar_wait_sleep(smem_u32(&b_full[sb]), (st / BST) & 1, 40)) {
-                    atomicExch(p.err, kDevErrFullWait);
+                const bool there = mbar_wait_bounded(smem_u32(&a_full[sa]), (st / AST) & 1) && mbar_wait_bounded(smem_u32(&b_full[sb]), (st / BST) & 1);
+                if (!__all_sync(0xffffffffu, there)) {
+                    if (lane == 0) atomicExch(p.err, kDevErrFullWait);
                     break;
                 }
                 tc_fence_after();
-                const uint32_t a0 = smem_u32(sm_a + (size_t)sa * Cfg::kABytes), b0 = smem_u32(sm_b + (size_t)sb * Cfg::kBBytes);
+                const uint64_t a0 = smem_desc_k128(smem_u32(sm_a + (size_t)sa * Cfg::kABytes)), b0 = smem_desc_k128(smem_u32(sm_b + (size_t)sb * Cfg::kBBytes));
 #pragma unroll 1
                 for (int j0 = 0; j0 < I8_BLOCKS; j0 += GROUP, ++gi) {
                     const int grp = gi & 1;
-                    if (gi >= 2 && !mbar_wait_sleep(smem_u32(&s_empty[grp]), ((gi >> 1) - 1) & 1, 40)) {  // the epilogue has drained this group's slots
-                        atomicExch(p.err, kDevErrMma);
+                    if (gi >= 2 && !__all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&s_empty[grp]), ((gi >> 1) - 1) & 1))) {  // the epilogue has drained this group's slots
+                        if (lane == 0) atomicExch(p.err, kDevErrMma);
                         ok = false;
                         break;
                     }
                     tc_fence_after();
+                    if (elect_one()) {
 #pragma unroll
-                    for (int jg = 0; jg < GROUP; ++jg) {
-                        const int j = j0 + jg;
-                        // block j: half j/4 of the tile (a [rows x 128 B] swizzled slab), 32 bytes of k inside the 128-byte row
-                        tc_mma_i8(tmem_base + (uint32_t)((grp * GROUP + jg) * NC), smem_desc_k128(a0 + (j >> 2) * (I8_ROWS * 128) + (j & 3) * 32),
-                                  smem_desc_k128(b0 + (j >> 2) * (NC * 128) + (j & 3) * 32), idesc);
+                        for (int jg = 0; jg < GROUP; ++jg) {
+                            const int j = j0 + jg;
+                            // block j: half j/4 of the tile (a [rows x 128 B] swizzled slab), 32 bytes of k inside the 128-byte row
+                            tc_mma_i8(tmem_base + (uint32_t)((grp * GROUP + jg) * NC), a0 + (uint64_t)((j >> 2) * (I8_ROWS * 128 / 16) + (j & 3) * 2),
+                                      b0 + (uint64_t)((j >> 2) * (NC * 128 / 16) + (j & 3) * 2), idesc);
+                        }
+                        tc_commit(smem_u32(&s_full[grp]));  // arrives when the group's MMAs (and all before) have completed
+                        if (j0 + GROUP >= I8_BLOCKS) {
+                            tc_commit(smem_u32(&a_empty[sa]));  // arrive when the chunk's MMAs have finished reading shared memory
+                            tc_commit(smem_u32(&b_empty[sb]));
+                        }
                     }
-                    tc_commit(smem_u32(&s_full[grp]));  // arrives when the group's MMAs (and all before) have completed
+                    __syncwarp();
                 }
-                if (!ok) break;
-                tc_commit(smem_u32(&a_empty[sa]));  // arrive when the chunk's MMAs have finished reading shared memory
-                tc_commit(smem_u32(&b_empty[sb]));
             }
         }
     } else if (warp >= Cfg::kWarpUnpack0 && warp < Cfg::kWarpEp0) {
@@ -362,39 +375,42 @@ __global__ void __launch_bounds__(I8Cfg<QT, NC>::kThreads, 1)
                 break;
             }
             // The thread's row of the stage, 144 / 272 bytes, in 16-byte loads: at this row pitch eight lanes' 16 bytes
-            // fall into distinct banks (32-bit loads would collide four ways).
-            constexpr int ROWW = Cfg::kRowChunk / 4;  // 36 / 68 words
-            uint32_t row[ROWW];
-            {
-                const uint4 *src = reinterpret_cast<const uint4 *>(sm_w + (size_t)sw * Cfg::kWBytes + (size_t)r * Cfg::kRowChunk);
-#pragma unroll
-                for (int i = 0; i < ROWW / 4; ++i) {
-                    const uint4 t = src[i];
-                    row[4 * i] = t.x, row[4 * i + 1] = t.y, row[4 * i + 2] = t.z, row[4 * i + 3] = t.w;
-                }
-            }
+            // fall into distinct banks (32-bit loads would collide four ways).  Q8_0 in two halves of four blocks (136 bytes,
+            // the second read from byte 128 on): the registers of a whole row are not there with sixteen epilogue warps.
+            constexpr int PASSES = QT == CQ_Q4_0 ? 1 : 2, BPP = I8_BLOCKS / PASSES;
             uint8_t *a_tile = sm_a + (size_t)sa * Cfg::kABytes;
             float *ws = sm_ws + (size_t)sa * (I8_BLOCKS * I8_ROWS);
 #pragma unroll
-            for (int j = 0; j < I8_BLOCKS; ++j) {
-                constexpr int HWB = Cfg::kBlockBytes / 2;  // 16-bit units per block: 9 / 17
-                const uint32_t dword = row[(HWB * j) / 2];
-                const uint32_t dbits = ((HWB * j) & 1) ? (dword >> 16) : (dword & 0xFFFFu);
-                ws[j * I8_ROWS + r] = __half2float(__ushort_as_half((unsigned short)dbits));
-                uint32_t o[8];
-                if (QT == CQ_Q4_0) {
-                    uint32_t q[4];
-                    row_words<4, ROWW>(row, HWB * j + 1, q);
+            for (int ps = 0; ps < PASSES; ++ps) {
+                uint32_t row[36];
+                const uint4 *src = reinterpret_cast<const uint4 *>(sm_w + (size_t)sw * Cfg::kWBytes + (size_t)r * Cfg::kRowChunk + ps * 128);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) o[i] = q[i] & 0x0F0F0F0Fu, o[4 + i] = (q[i] >> 4) & 0x0F0F0F0Fu;
-                } else {
-                    row_words<8, ROWW>(row, HWB * j + 1, o);
+                for (int i = 0; i < 9; ++i) {
+                    const uint4 t = src[i];
+                    row[4 * i] = t.x, row[4 * i + 1] = t.y, row[4 * i + 2] = t.z, row[4 * i + 3] = t.w;
                 }
-                // block j -> bytes [32 (j & 3), +32) of the 128-byte row of half j >> 2; 16-byte chunk c sits at c ^ (r & 7)
-                uint8_t *dst = a_tile + (j >> 2) * (I8_ROWS * 128) + r * 128;
-                const int c = 2 * (j & 3);
-                *reinterpret_cast<uint4 *>(dst + ((c ^ (r & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
-                *reinterpret_cast<uint4 *>(dst + (((c + 1) ^ (r & 7)) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
+#pragma unroll
+                for (int jp = 0; jp < BPP; ++jp) {
+                    constexpr int HWB = Cfg::kBlockBytes / 2;  // 16-bit units per block: 9 / 17
+                    const int j = ps * BPP + jp, hw = HWB * jp + (ps ? 4 : 0);  // (byte 136 is 8 bytes past byte 128)
+                    const uint32_t dword = row[hw / 2];
+                    const uint32_t dbits = (hw & 1) ? (dword >> 16) : (dword & 0xFFFFu);
+                    ws[j * I8_ROWS + r] = __half2float(__ushort_as_half((unsigned short)dbits));
+                    uint32_t o[8];
+                    if (QT == CQ_Q4_0) {
+                        uint32_t q[4];
+                        row_words<4, 36>(row, hw + 1, q);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) o[i] = q[i] & 0x0F0F0F0Fu, o[4 + i] = (q[i] >> 4) & 0x0F0F0F0Fu;
+                    } else {
+                        row_words<8, 36>(row, hw + 1, o);
+                    }
+                    // block j -> bytes [32 (j & 3), +32) of the 128-byte row of half j >> 2; 16-byte chunk c sits at c ^ (r & 7)
+                    uint8_t *dst = a_tile + (j >> 2) * (I8_ROWS * 128) + r * 128;
+                    const int c = 2 * (j & 3);
+                    *reinterpret_cast<uint4 *>(dst + ((c ^ (r & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+                    *reinterpret_cast<uint4 *>(dst + (((c + 1) ^ (r & 7)) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
+                }
             }
             fence_proxy_async();  // the A tile is read by the tensor core's asynchronous proxy
             __syncwarp();
@@ -411,9 +427,11 @@ __global__ void __launch_bounds__(I8Cfg<QT, NC>::kThreads, 1)
         const int lcol0 = chalf * LPW;                       // first logical column of this warp inside the launch
         const int r = quarter * 32 + lane;
         pdl_wait_prior();  // y and the partial tiles may still be read by earlier kernels
-        float acc[LPW];
+        static_assert(LPW % 8 == 0, "a piece is whole pairs of columns");
+        uint64_t acc2[LPW / 2];  // Q8_1 columns: two each
+        float acc[LPW];          // plane columns
 #pragma unroll
-        for (int i = 0; i < LPW; ++i) acc[i] = 0.0f;
+        for (int i = 0; i < LPW; ++i) acc[i] = 0.0f, acc2[i / 2] = 0;
         int st = 0, gi = 0;  // chunks and groups of blocks drained so far
         bool ok = true, first_seg = true;
         for (int g = g0; g < g1 && ok;) {
@@ -450,12 +468,17 @@ __global__ void __launch_bounds__(I8Cfg<QT, NC>::kThreads, 1)
                         const int j = j0 + e / PPB, cb = e % PPB;
                         const float dw = ws[j * I8_ROWS + r];
                         if (MODE == 1) {
+                            // Two columns per instruction.  The integers become floats by an addition (|sumi| < 2^22 sits exactly
+                            // in the mantissa of 1.5 * 2^23 + sumi): the conversion unit passes 16 lanes a cycle and SM and was
+                            // what this loop waited for (n 11008, k 4096, 100 columns of Q8_0: 82.5 -> 56.3 us, the same bits).
+                            const uint64_t dw2 = dup2(dw), magic = dup2(-12582912.0f);
 #pragma unroll
-                            for (int i = 0; i < 16; ++i) {
-                                const float2 sc = xs[j * NCL + lcol0 + cb * 16 + i];  // (d8, s8): the same address in every lane
-                                const float sumi = (float)(int)v[i];
-                                if (QT == CQ_Q4_0) acc[cb * 16 + i] = fmaf(dw, fmaf(sumi, sc.x, -8.0f * sc.y), acc[cb * 16 + i]);
-                                else acc[cb * 16 + i] = fmaf(dw * sc.x, sumi, acc[cb * 16 + i]);
+                            for (int i = 0; i < 8; ++i) {
+                                const float4 sc = reinterpret_cast<const float4 *>(xs)[(j * NCL + lcol0 + cb * 16) / 2 + i];  // (d8, d8', -8 s8, -8 s8'): the same address in every lane
+                                const uint64_t f = add2(pack2(__uint_as_float(v[2 * i] + 0x4B400000u), __uint_as_float(v[2 * i + 1] + 0x4B400000u)), magic);
+                                uint64_t &a = acc2[cb * 8 + i];
+                                if (QT == CQ_Q4_0) a = fma2(dw2, fma2(f, pack2(sc.x, sc.y), pack2(sc.z, sc.w)), a);
+                                else a = fma2(mul2(dw2, pack2(sc.x, sc.y)), f, a);
                             }
                         } else {
 #pragma unroll
@@ -466,17 +489,27 @@ __global__ void __launch_bounds__(I8Cfg<QT, NC>::kThreads, 1)
                             }
                         }
                     };
-                    uint32_t va[16], vb[16];
-                    fetch(va, 0);
-                    tmem_wait_ld();
+                    if (EPW >= 16) {
 #pragma unroll
-                    for (int u = 0; u < PIECES / 2; ++u) {
-                        fetch(vb, 2 * u + 1);
-                        consume(va, 2 * u);
+                        for (int e = 0; e < PIECES; ++e) {
+                            uint32_t v[16];
+                            fetch(v, e);
+                            tmem_wait_ld();
+                            consume(v, e);
+                        }
+                    } else {
+                        uint32_t va[16], vb[16];
+                        fetch(va, 0);
                         tmem_wait_ld();
-                        if (2 * u + 2 < PIECES) fetch(va, 2 * u + 2);
-                        consume(vb, 2 * u + 1);
-                        tmem_wait_ld();
+#pragma unroll
+                        for (int u = 0; u < PIECES / 2; ++u) {
+                            fetch(vb, 2 * u + 1);
+                            consume(va, 2 * u);
+                            tmem_wait_ld();
+                            if (2 * u + 2 < PIECES) fetch(va, 2 * u + 2);
+                            consume(vb, 2 * u + 1);
+                            tmem_wait_ld();
+                        }
                     }
                     // every piece of the group is in registers or already used: its slots may be overwritten
                     tc_fence_before();
@@ -497,15 +530,19 @@ __global__ void __launch_bounds__(I8Cfg<QT, NC>::kThreads, 1)
 #pragma unroll
             for (int i = 0; i < LPW; ++i) {
                 const int lc = lcol0 + i;
+                float lo, hi;
+                unpack2(acc2[i / 2], lo, hi);
+                const float v = MODE == 0 ? acc[i] : (i & 1) ? hi : lo;
                 if (lc < p.ncols) {
                     if (direct) {
-                        if (row < p.n) p.y[(int64_t)lc * p.ldy + row] = acc[i];
+                        if (row < p.n) p.y[(int64_t)lc * p.ldy + row] = v;
                     } else {
-                        p.part[((int64_t)(2 * blockIdx.x + (first_seg ? 0 : 1)) * p.ncols + lc) * I8_ROWS + r] = acc[i];
+                        p.part[((int64_t)(2 * blockIdx.x + (first_seg ? 0 : 1)) * p.ncols + lc) * I8_ROWS + r] = v;
                     }
                 }
-                acc[i] = 0.0f;
             }
+#pragma unroll
+            for (int i = 0; i < LPW; ++i) acc[i] = 0.0f, acc2[i / 2] = 0;
             first_seg = false;
         }
     }
@@ -590,10 +627,10 @@ template <int QT, int MODE, int NC>
 cq_status run_i8(cq_ctx *ctx, const CUtensorMap &tmW, const CUtensorMap &tmX, const I8Params &p, unsigned ctas) {
     static thread_local int configured = -1;
     if (configured != ctx->device) {
-        CQ_CUDA(ctx, cudaFuncSetAttribute(qgemm_i8_kernel<QT, MODE, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)I8Cfg<QT, NC>::kSmem));
+        CQ_CUDA(ctx, cudaFuncSetAttribute(qgemm_i8_kernel<QT, MODE, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)I8Cfg<QT, MODE, NC>::kSmem));
         configured = ctx->device;
     }
-    return i8_launch_chained(ctx, qgemm_i8_kernel<QT, MODE, NC>, dim3(ctas), dim3(I8Cfg<QT, NC>::kThreads), I8Cfg<QT, NC>::kSmem, tmW, tmX, p);
+    return i8_launch_chained(ctx, qgemm_i8_kernel<QT, MODE, NC>, dim3(ctas), dim3(I8Cfg<QT, MODE, NC>::kThreads), I8Cfg<QT, MODE, NC>::kSmem, tmW, tmX, p);
 }
 
 template <int QT, int MODE>

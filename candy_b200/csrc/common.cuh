@@ -179,6 +179,10 @@ cq_status launch_gemv_mma_f16(cq_ctx *ctx, int order, const float *x, int64_t m,
                               float *y, int64_t ldy);
 cq_status launch_qgemm_i8(cq_ctx *ctx, int qtype, int order, int mode, const float *x, int64_t m, int64_t k, int64_t ldx, const void *w, int64_t n,
                           float *y, int64_t ldy);
+// CQ_ACT_F32 in plain f32, any m, any k % 32 == 0 (gemv_f32.cu): the formats and alignments it takes.
+bool gemv_f32_supported(int qtype, const void *w, const float *x, const float *y);
+cq_status launch_gemv_f32(cq_ctx *ctx, int qtype, int order, const float *x, int64_t m, int64_t k, int64_t ldx, const void *w, int64_t n, float *y,
+                          int64_t ldy);
 // Batches on CTA pairs, raw blocks dequantized into tensor memory (gemm_pair_tmem.cu): split = CQ_ACT_F32 by sums of two
 // f16 numbers, otherwise CQ_ACT_F16.
 bool gemm_pair_tmem_supported(int qtype, int64_t k, const void *w);

@@ -519,6 +519,9 @@ bool make_map(CUtensorMap *map, const void *base, int64_t rows, int64_t k, int b
 
 cq_status launch_gemm(cq_ctx *ctx, int qtype, int order, int actmode, const float *x, int64_t m, int64_t k, int64_t ldx,
                       const void *w, int64_t n, float *y, int64_t ldy) {
+    if (actmode == CQ_ACT_F32 && ctx->tune.gemv_variant == 0 && !ctx->tune.force_simple && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && ldx % 4 == 0 &&
+        gemv_f32_supported(qtype, w, x, y) && (cq_is_more_format(qtype) || cq_is_k_format(qtype) || !qgemm_i8_supported(qtype, k, w, x, ldx)))
+        return launch_gemv_f32(ctx, qtype, order, x, m, k, ldx, w, n, y, ldy);
     if (actmode != CQ_ACT_F16) {
         // f32 / Q8_1 activation numerics for m > 8: the decode kernels, eight rows at a time
         // (weights are re-read once per eight rows; the tensor-core path is CQ_ACT_F16).

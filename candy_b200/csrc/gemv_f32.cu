@@ -1,0 +1,323 @@
+// CQ_ACT_F32 products in plain f32: y[m, n] = sum_k x[m, k] W[n, k], weights dequantized in registers, f32 multiplies and
+// adds.  Serves the calls that the block-integer kernels do not take: Q4_0 / Q8_0 rows whose length is not a multiple of 256
+// (or pointers without 16-byte alignment), two and more rows of Q4_1 / Q5_0 / Q5_1, and Q4_K / Q5_K / Q6_K.
+//
+// What bounds it: the instructions that turn bits into f32 (about 2.5 per weight with the multiply by the scale), then the
+// multiply-adds themselves (one per weight and row of x).  So a weight is decoded once for all M rows of x, and an x value
+// read from shared memory is used for R weight rows:
+//   * a CTA of sixteen warps stays on its SM; the x rows (or, if they do not fit, a chunk of k at a time) lie in shared
+//     memory for all of its weight rows, 36 words per 32-block: lanes that read 16 bytes each hit distinct banks;
+//   * a warp takes R weight rows; lane l owns blocks l, l + 32, ...: neighbouring lanes read neighbouring blocks, as 32-bit
+//     words of memory shifted into place (blocks are 2-byte aligned), all R rows' words in flight before the first is used;
+//   * the R x M sums are exchanged between the lanes by a butterfly that halves their number at each step.
+// The kernels before it read the blocks byte by byte and x from global memory, one weight row per warp: n 11008, k 4192,
+// Q4_0, us, before -> now: 1 row 185 -> 21, 8 rows 1387 -> 42,
+// 64 rows 11097 -> 310.  Q4_K, k 4096: 1 row 52 -> 16, 8 rows 230 -> 37; Q6_K 54 -> 23 and 241 -> 41.
+#include "common.cuh"
+
+namespace {
+
+constexpr int GF_WARPS = 16, GF_THREADS = 32 * GF_WARPS;
+constexpr int GF_PITCH = 36;                    // words per 32-block of x in shared memory
+constexpr size_t GF_SMEM = 200 << 10;
+
+__device__ __forceinline__ uint32_t ldw(const uint8_t *p) { return __ldg(reinterpret_cast<const uint32_t *>(p)); }
+
+// N words that start `skip` (2 or 0) bytes past p, p 2-byte aligned.  Reads whole aligned words: at most two bytes before
+// or after the wanted ones, inside the same four.
+template <int N>
+__device__ __forceinline__ void words_from(const uint8_t *p, uint32_t (&out)[N]) {
+    const uint32_t odd = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 2);
+    const uint8_t *q = p - odd;
+    uint32_t v[N + 1];
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = ldw(q + 4 * i);
+    v[N] = odd ? ldw(q + 4 * N) : 0u;
+#pragma unroll
+    for (int i = 0; i < N; ++i) out[i] = __funnelshift_r(v[i], v[i + 1], 8 * odd);
+}
+__device__ __forceinline__ float half_at(const uint8_t *p) { return __half2float(__ushort_as_half(__ldg(reinterpret_cast<const unsigned short *>(p)))); }
+
+// byte i of w as a float, minus `off` (whole numbers below 2^23: the sum 2^23 + byte and the difference are exact)
+__device__ __forceinline__ float byte_f(uint32_t w, int i, float off) {
+    return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440 + i)) - (8388608.0f + off);
+}
+
+// One 32-value block of a weight row.  After load(): value groups g = 0..7 of four consecutive k from pos(g) on are bytes of
+// word(g); value = scale(g) * (byte - kOff) - min.
+template <int QT, int ORDER>
+struct Blk {
+    static constexpr bool kNib = QT == CQ_Q4_0 || QT == CQ_Q4_1 || QT == CQ_Q5_0 || QT == CQ_Q5_1;  // nibbles kept packed, a group's bytes made on use
+    static constexpr bool kMin = QT == CQ_Q4_1 || QT == CQ_Q5_1 || QT == CQ_Q4_K || QT == CQ_Q5_K;
+    static constexpr bool kFive = QT == CQ_Q5_0 || QT == CQ_Q5_1;
+    static constexpr float kOff = QT == CQ_Q4_0 ? 8.0f : QT == CQ_Q5_0 ? 16.0f : QT == CQ_Q8_0 ? 128.0f : QT == CQ_Q6_K ? 32.0f : 0.0f;
+    uint32_t q[kNib ? 4 : 8];
+    uint32_t qh;       // Q5_0 / Q5_1: the fifth bits
+    float d[QT == CQ_Q6_K ? 2 : 1], mn;
+
+    // wr: the row's first byte, b: the block's number in the row
+    __device__ __forceinline__ void load(const uint8_t *wr, int b) {
+        if (QT == CQ_Q4_0) {
+            const uint8_t *p = wr + (int64_t)b * 18;
+            d[0] = half_at(p);
+            words_from<4>(p + 2, reinterpret_cast<uint32_t(&)[4]>(q));
+        } else if (QT == CQ_Q8_0) {
+            const uint8_t *p = wr + (int64_t)b * 34;
+            d[0] = half_at(p);
+            words_from<8>(p + 2, reinterpret_cast<uint32_t(&)[8]>(q));
+#pragma unroll
+            for (int i = 0; i < 8; ++i) q[i] ^= 0x80808080u;
+        } else if (QT == CQ_Q5_0) {
+            const uint8_t *p = wr + (int64_t)b * 22;
+            d[0] = half_at(p);
+            uint32_t v[5];
+            words_from<5>(p + 2, v);
+            qh = v[0];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) q[i] = v[1 + i];
+        } else if (QT == CQ_Q4_1 || QT == CQ_Q5_1) {
+            const uint8_t *p = wr + (int64_t)b * (QT == CQ_Q4_1 ? 20 : 24);
+            const uint32_t dm = ldw(p);
+            d[0] = __half2float(__ushort_as_half((unsigned short)(dm & 0xFFFFu)));
+            mn = -__half2float(__ushort_as_half((unsigned short)(dm >> 16)));
+            if (QT == CQ_Q5_1) qh = ldw(p + 4);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) q[i] = ldw(p + (QT == CQ_Q4_1 ? 4 : 8) + 4 * i);
+        } else if (QT == CQ_Q4_K || QT == CQ_Q5_K) {
+            // sub-block j of a super-block: nibble j & 1 of qs[32 (j >> 1) ..], scale pair j (quantized.cu:994-1006, :1008-1082)
+            const int j = b & 7, h = j & 1;
+            const uint4 *p = reinterpret_cast<const uint4 *>(wr + (int64_t)(b >> 3) * (QT == CQ_Q4_K ? 144 : 176));
+            const uint4 head = __ldg(p);
+            const uint4 *qs = p + (QT == CQ_Q4_K ? 1 : 3) + 2 * (j >> 1);
+            const uint4 a = __ldg(qs), c = __ldg(qs + 1);
+            const uint32_t s0 = head.y, s1 = head.z, s2 = head.w;  // scale bytes 0-3, 4-7, 8-11
+            const int sh = 8 * (j & 3);
+            uint32_t sc, m;
+            if (j < 4) {
+                sc = (s0 >> sh) & 63;
+                m = (s1 >> sh) & 63;
+            } else {
+                sc = ((s2 >> sh) & 15) | (((s0 >> (sh + 6)) & 3) << 4);
+                m = ((s2 >> (sh + 4)) & 15) | (((s1 >> (sh + 6)) & 3) << 4);
+            }
+            d[0] = __half2float(__ushort_as_half((unsigned short)(head.x & 0xFFFFu))) * (float)sc;
+            mn = __half2float(__ushort_as_half((unsigned short)(head.x >> 16))) * (float)m;
+            const uint32_t w[8] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) q[i] = (w[i] >> (4 * h)) & 0x0F0F0F0Fu;
+            if (QT == CQ_Q5_K) {
+                const uint4 e = __ldg(p + 1), f = __ldg(p + 2);
+                const uint32_t hb[8] = {e.x, e.y, e.z, e.w, f.x, f.y, f.z, f.w};
+#pragma unroll
+                for (int i = 0; i < 8; ++i) q[i] |= ((hb[i] >> j) & 0x01010101u) << 4;
+            }
+        } else {
+            // Q6_K, values 128 ip + 32 t + l (quantized.cu:1099-1123): ql[64 ip + 32 (t & 1) + l] nibble t >> 1, two bits of qh[32 ip + l]
+            const int ip = (b >> 2) & 1, t = b & 3;
+            const uint8_t *p = wr + (int64_t)(b >> 3) * 210;
+            uint32_t lo[8], hi[8];
+            words_from<8>(p + 64 * ip + 32 * (t & 1), lo);
+            words_from<8>(p + 128 + 32 * ip, hi);
+            const uint32_t s = __ldg(reinterpret_cast<const unsigned short *>(p + 192 + 8 * ip + 2 * t));
+            const float dd = half_at(p + 208);
+            d[0] = dd * (float)(int)(signed char)(s & 0xFF);
+            d[QT == CQ_Q6_K ? 1 : 0] = dd * (float)(int)(signed char)(s >> 8);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) q[i] = ((lo[i] >> (4 * (t >> 1))) & 0x0F0F0F0Fu) | (((hi[i] >> (2 * t)) & 0x03030303u) << 4);
+        }
+    }
+    static __device__ __forceinline__ constexpr int pos(int g) {
+        // packed nibbles: interleaved order has word i's values at 8 i .., split order its low nibbles at 4 i .., the high ones 16 further
+        return !kNib || ORDER == CQ_ORDER_GO_INTERLEAVED ? 4 * g : 4 * (g >> 1) + 16 * (g & 1);
+    }
+    __device__ __forceinline__ void values(int g, float (&v)[4]) const {
+        uint32_t w;
+        if (!kNib) {
+            w = q[g];
+        } else if (ORDER == CQ_ORDER_GO_INTERLEAVED) {
+            const uint32_t two = (q[g >> 1] >> (16 * (g & 1))) & 0xFFFFu;  // bytes (n0 n1) (n2 n3)
+            const uint32_t spread = __byte_perm(two, 0, 0x1100);           // n0n1 n0n1 n2n3 n2n3
+            w = (spread & 0x000F000Fu) | ((spread >> 4) & 0x0F000F00u);
+        } else {
+            w = (q[g >> 1] >> (4 * (g & 1))) & 0x0F0F0F0Fu;
+            if (kFive) w |= ((((qh >> pos(g)) & 15u) * 0x00204081u) & 0x01010101u) << 4;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = d[QT == CQ_Q6_K ? (g >> 2) : 0] * byte_f(w, i, kOff);
+    }
+};
+
+struct GfParams {
+    const uint8_t *w;
+    const float *x, *bias;
+    float *y;
+    int64_t n, ldx, ldy, row_bytes;
+    int m, nb, chunk;  // blocks per row, and per chunk of k that lies in shared memory
+};
+
+template <int QT, int ORDER, int M, int R>
+__global__ void __launch_bounds__(GF_THREADS, 1) gemv_f32_kernel(const GfParams p) {
+    extern __shared__ __align__(16) float gf_x[];  // [M][chunk][36], then [M][chunk] block sums
+    float *xsum = gf_x + (size_t)M * p.chunk * GF_PITCH;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int m0 = blockIdx.y * M, rows = min(M, p.m - m0);
+    const float *x = p.x + (int64_t)m0 * p.ldx;
+    const int64_t groups = (p.n + R - 1) / R;
+    for (int b0 = 0; b0 < p.nb; b0 += p.chunk) {
+        const int cnt = min(p.chunk, p.nb - b0);
+        __syncthreads();
+        for (int r = 0; r < M; ++r)
+            for (int i = threadIdx.x; i < cnt * kQK; i += GF_THREADS)
+                gf_x[(r * p.chunk + (i >> 5)) * GF_PITCH + (i & 31)] = r < rows ? x[(int64_t)r * p.ldx + (int64_t)b0 * kQK + i] : 0.0f;
+        __syncthreads();
+        if (Blk<QT, ORDER>::kMin) {
+            for (int i = threadIdx.x; i < M * cnt; i += GF_THREADS) {
+                const int r = i / cnt, b = i - r * cnt;
+                const float4 *v = reinterpret_cast<const float4 *>(gf_x + (r * p.chunk + b) * GF_PITCH);
+                float s = 0.0f;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) s += (v[j].x + v[j].y) + (v[j].z + v[j].w);
+                xsum[r * p.chunk + b] = s;
+            }
+            __syncthreads();
+        }
+        for (int64_t grp = (int64_t)warp * gridDim.x + blockIdx.x; grp < groups; grp += (int64_t)GF_WARPS * gridDim.x) {
+            float acc[R * M];
+#pragma unroll
+            for (int i = 0; i < R * M; ++i) acc[i] = 0.0f;
+            const uint8_t *wr[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int64_t row = grp * R + r;
+                wr[r] = p.w + (row < p.n ? row : p.n - 1) * p.row_bytes;
+            }
+            for (int b = lane; b < cnt; b += 32) {
+                Blk<QT, ORDER> blk[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) blk[r].load(wr[r], b0 + b);
+                if (Blk<QT, ORDER>::kMin) {
+#pragma unroll
+                    for (int i = 0; i < M; ++i) {
+                        const float s = xsum[i * p.chunk + b];
+#pragma unroll
+                        for (int r = 0; r < R; ++r) acc[r * M + i] = fmaf(-blk[r].mn, s, acc[r * M + i]);
+                    }
+                }
+#pragma unroll
+                for (int g = 0; g < 8; ++g) {
+                    float v[R][4];
+#pragma unroll
+                    for (int r = 0; r < R; ++r) blk[r].values(g, v[r]);
+#pragma unroll
+                    for (int i = 0; i < M; ++i) {
+                        const float4 t = *reinterpret_cast<const float4 *>(gf_x + (i * p.chunk + b) * GF_PITCH + Blk<QT, ORDER>::pos(g));
+#pragma unroll
+                        for (int r = 0; r < R; ++r)
+                            acc[r * M + i] = fmaf(v[r][0], t.x, fmaf(v[r][1], t.y, fmaf(v[r][2], t.z, fmaf(v[r][3], t.w, acc[r * M + i]))));
+                    }
+                }
+            }
+            // lanes exchange: at each step half of the sums that a lane holds go to its partner, the partner's come here
+            int idx = 0;
+#pragma unroll
+            for (int step = 0; step < 5; ++step) {
+                const int off = 16 >> step, left = (R * M) >> step;  // sums per lane before this step
+                if (left >= 2) {
+                    const bool up = lane & off;
+#pragma unroll
+                    for (int i = 0; i < left / 2; ++i) {
+                        const float send = up ? acc[i] : acc[i + left / 2], keep = up ? acc[i + left / 2] : acc[i];
+                        acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+                    }
+                    if (up) idx += left / 2;
+                } else {
+                    acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], off);
+                }
+            }
+            constexpr int kDup = 32 / (R * M);  // lanes that end up with the same sum
+            const int64_t row = grp * R + idx / M;
+            const int xr = idx % M;
+            if (lane % kDup == 0 && row < p.n && xr < rows) {
+                float *dst = p.y + (int64_t)(m0 + xr) * p.ldy + row;
+                float v = b0 > 0 ? *dst + acc[0] : acc[0];  // (the same lane wrote it in the chunk before)
+                if (p.bias && b0 + p.chunk >= p.nb) v += p.bias[row];
+                *dst = v;
+            }
+        }
+    }
+}
+
+template <int QT, int ORDER, int M, int R>
+cq_status gf_run(cq_ctx *ctx, GfParams p) {
+    auto kern = gemv_f32_kernel<QT, ORDER, M, R>;
+    static thread_local int configured = -1;
+    if (configured != ctx->device) {
+        CQ_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GF_SMEM));
+        configured = ctx->device;
+    }
+    const int fit = (int)(GF_SMEM / ((size_t)M * (GF_PITCH + 1) * 4));
+    const int parts = (p.nb + fit - 1) / fit;
+    p.chunk = parts == 1 ? p.nb : (((p.nb + parts - 1) / parts + 31) & ~31) <= fit ? (((p.nb + parts - 1) / parts + 31) & ~31) : (fit & ~31);
+    const size_t smem = (size_t)M * p.chunk * (GF_PITCH + 1) * 4;
+    const int64_t groups = (p.n + R - 1) / R, want = (groups + GF_WARPS - 1) / GF_WARPS;
+    const dim3 grid((unsigned)(want < ctx->sm_count ? want : ctx->sm_count), (unsigned)((p.m + M - 1) / M));
+    kern<<<grid, GF_THREADS, smem, ctx->stream>>>(p);
+    CQ_CUDA(ctx, cudaGetLastError());
+    return CQ_OK;
+}
+
+template <int QT, int ORDER, int M>
+cq_status gf_rows(cq_ctx *ctx, const GfParams &p) {
+    // four weight rows per warp where that still gives every warp of the device one; else one, so that small matrices spread
+    constexpr int R = M == 8 && (QT == CQ_Q8_0 || QT == CQ_Q5_K || QT == CQ_Q4_K || QT == CQ_Q6_K) ? 2 : 4;  // (whole bytes: more registers per row)
+    if (p.n >= (int64_t)R * GF_WARPS * ctx->sm_count / 2) return gf_run<QT, ORDER, M, R>(ctx, p);
+    return gf_run<QT, ORDER, M, 1>(ctx, p);
+}
+
+template <int QT, int ORDER>
+cq_status gf_go(cq_ctx *ctx, const GfParams &p) {
+    if (p.m == 1) return gf_rows<QT, ORDER, 1>(ctx, p);
+    if (p.m == 2) return gf_rows<QT, ORDER, 2>(ctx, p);
+    if (p.m <= 4) return gf_rows<QT, ORDER, 4>(ctx, p);
+    return gf_rows<QT, ORDER, 8>(ctx, p);
+}
+
+}  // namespace
+
+bool gemv_f32_supported(int qtype, const void *w, const float *x, const float *y) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(w);
+    if ((reinterpret_cast<uintptr_t>(x) & 3) || (reinterpret_cast<uintptr_t>(y) & 3)) return false;
+    switch (qtype) {
+        case CQ_Q4_0: case CQ_Q8_0: case CQ_Q5_0: case CQ_Q6_K: return (a & 1) == 0;
+        case CQ_Q4_1: case CQ_Q5_1: return (a & 3) == 0;
+        case CQ_Q4_K: case CQ_Q5_K: return (a & 15) == 0;
+        default: return false;
+    }
+}
+
+cq_status launch_gemv_f32(cq_ctx *ctx, int qtype, int order, const float *x, int64_t m, int64_t k, int64_t ldx, const void *w, int64_t n, float *y,
+                          int64_t ldy) {
+    GfParams p = {};
+    p.w = static_cast<const uint8_t *>(w), p.x = x, p.y = y, p.bias = ctx->bias;
+    p.n = n, p.ldx = ldx, p.ldy = ldy, p.nb = (int)(k / kQK);
+    p.row_bytes = (int64_t)cq_blocks_bytes(qtype, 1, k);
+    const bool inter = order == CQ_ORDER_GO_INTERLEAVED;
+    cq_status s = CQ_OK;
+    for (int64_t r = 0; r < m && s == CQ_OK; r += 8 * 32768) {  // (a grid is at most 65535 high)
+        p.m = (int)(m - r < 8 * 32768 ? m - r : 8 * 32768);
+        p.x = x + r * ldx, p.y = y + r * ldy;
+        switch (qtype) {
+            case CQ_Q4_0: s = inter ? gf_go<CQ_Q4_0, 0>(ctx, p) : gf_go<CQ_Q4_0, 1>(ctx, p); break;
+            case CQ_Q8_0: s = gf_go<CQ_Q8_0, 0>(ctx, p); break;
+            case CQ_Q4_1: s = inter ? gf_go<CQ_Q4_1, 0>(ctx, p) : gf_go<CQ_Q4_1, 1>(ctx, p); break;
+            case CQ_Q5_0: s = gf_go<CQ_Q5_0, 1>(ctx, p); break;
+            case CQ_Q5_1: s = gf_go<CQ_Q5_1, 1>(ctx, p); break;
+            case CQ_Q4_K: s = gf_go<CQ_Q4_K, 1>(ctx, p); break;
+            case CQ_Q5_K: s = gf_go<CQ_Q5_K, 1>(ctx, p); break;
+            case CQ_Q6_K: s = gf_go<CQ_Q6_K, 1>(ctx, p); break;
+            default: return cq_fail(ctx, CQ_ERR_UNSUPPORTED, "gemv: unknown block format");
+        }
+    }
+    if (s == CQ_OK && p.bias) ctx->bias_done = true;
+    return s;
+}

@@ -1746,6 +1746,7 @@ cq_status gemv_dispatch(cq_ctx *ctx, int actmode, const float *x, int64_t m, int
     }
     if (ctx->push.world > 0) return cq_fail(ctx, CQ_ERR_UNSUPPORTED, "pushing GEMV needs a shape the streaming kernel takes (k % 256 == 0, aligned pointers)");
     if (ctx->fuse.on) return cq_fail(ctx, CQ_ERR_UNSUPPORTED, "fused linear needs a shape the streaming kernel takes (k % 256 == 0, aligned pointers, an even row-group count for the pairing epilogue)");
+    if (!ctx->tune.force_simple && gemv_f32_supported(QT, w, x, y)) return launch_gemv_f32(ctx, QT, ORDER, x, m, k, ldx, w, n, y, ldy);
     return run_simple<QT, ORDER>(ctx, w, x, y, m, n, nb, ldx, ldy);
 }
 
@@ -1780,11 +1781,16 @@ cq_status launch_gemv(cq_ctx *ctx, int qtype, int order, int actmode, const floa
         if (actmode == CQ_ACT_F32) {
             cq_status s = CQ_OK;
             bool taken;
+            // One row: the streaming kernel (n 11008, k 4096: 9.0 us for Q4_1).  It would read the weights once per row, so two and
+            // more (8 rows: 66 us), and rows that it cannot stream, run in plain f32 with one pass for eight (33 us; 2 rows 16.7 / 17.4).
+            const bool plain = !ctx->tune.force_simple && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && ldx % 4 == 0 && gemv_f32_supported(qtype, w, x, y);
+            if (plain && m >= 2) return launch_gemv_f32(ctx, qtype, order, x, m, k, ldx, w, n, y, ldy);
             if (qtype == CQ_Q4_1 && order == CQ_ORDER_GO_INTERLEAVED) taken = try_stream_more<CQ_Q4_1, 0>(ctx, x, m, k, ldx, w, n, y, ldy, s);
             else if (qtype == CQ_Q4_1) taken = try_stream_more<CQ_Q4_1, 1>(ctx, x, m, k, ldx, w, n, y, ldy, s);
             else if (qtype == CQ_Q5_0) taken = try_stream_more<CQ_Q5_0, 1>(ctx, x, m, k, ldx, w, n, y, ldy, s);
             else taken = try_stream_more<CQ_Q5_1, 1>(ctx, x, m, k, ldx, w, n, y, ldy, s);
             if (taken) return s;
+            if (plain) return launch_gemv_f32(ctx, qtype, order, x, m, k, ldx, w, n, y, ldy);
         }
         return launch_gemv_more(ctx, qtype, order, actmode, x, m, k, ldx, w, n, y, ldy);
     }

@@ -229,7 +229,8 @@ cq_status launch_gemv_k(cq_ctx *ctx, int qtype, int actmode, const float *x, int
                         int64_t ldy) {
     if (actmode != CQ_ACT_F32) return cq_fail(ctx, CQ_ERR_UNSUPPORTED, "the K formats take f32 (GEMV) or f16 (GEMM) activations, not Q8_1");
     if ((reinterpret_cast<uintptr_t>(x) & 15) != 0 || (ldx & 3) != 0) return cq_fail(ctx, CQ_ERR_INVALID_ARG, "x must be 16-byte aligned with ldx % 4 == 0");
-    constexpr int kWarps = 8;
+    if (gemv_f32_supported(qtype, w, x, y)) return launch_gemv_f32(ctx, qtype, CQ_ORDER_GGML_SPLIT, x, m, k, ldx, w, n, y, ldy);
+    constexpr int kWarps = 8;  // Q2_K, Q3_K, and blocks at odd addresses
     const unsigned grid = (unsigned)((n + kWarps - 1) / kWarps);
     const uint8_t *wb = static_cast<const uint8_t *>(w);
     const int nsb = (int)(k / 256);

@@ -1,0 +1,130 @@
+"""Rows that are not multiples of 256 values, and the formats without integer kernels: plain f32 products (gemv_f32.cu) and,
+for CQ_ACT_Q8_1 / CQ_ACT_F16, padded copies on the fast routes.  Against f64, resp. the oracle's Q8_1 arithmetic."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from candy_b200 import abi
+from candy_b200.backend import ACT_F16, ACT_F32, ACT_Q8_1, RawBuffer
+from oracle import oracle_c as oc
+
+pytestmark = pytest.mark.gpu
+at = lambda p, off: C.c_void_p(p.value + off)  # noqa: E731
+
+
+def run(device, qt, order, act, blocks, n, x, ldx=None, bias=None, w_off=0, x_off=0):
+    m, k = x.shape
+    ldx = ldx or k
+    xs = np.full((m, ldx), 3.0, dtype=np.float32)
+    xs[:, :k] = x
+    wb, xb = RawBuffer(device, blocks.nbytes + w_off), RawBuffer(device, xs.nbytes + x_off)
+    lib, ctx = device._lib, device.ctx
+    abi.check(ctx, lib.cq_memcpy_h2d(ctx, at(wb.ptr, w_off), blocks.ctypes.data_as(C.c_void_p), blocks.nbytes), "w")
+    abi.check(ctx, lib.cq_memcpy_h2d(ctx, at(xb.ptr, x_off), xs.ctypes.data_as(C.c_void_p), xs.nbytes), "x")
+    yd = device.storage_from_slice(np.full((m, n + 1), -5.0, dtype=np.float32))
+    bd = device.storage_from_slice(bias) if bias is not None else None
+    abi.check(ctx, lib.cq_qlinear(ctx, qt, order, act, at(xb.ptr, x_off), m, k, ldx, at(wb.ptr, w_off), n, bd.ptr if bd else None, yd.ptr, n + 1), "linear")
+    device.synchronize()
+    y = yd.data().reshape(m, n + 1)
+    assert (y[:, n] == -5.0).all()
+    return y[:, :n]
+
+
+def blocks_of(device, qt, order, n, k, seed):
+    rng = np.random.default_rng(seed)
+    if qt in abi.K_BLOCK_BYTES:
+        b = rng.integers(0, 256, size=(n * (k // 256), abi.K_BLOCK_BYTES[qt]), dtype=np.uint8)
+        for off in ([208] if qt == abi.Q6_K else [0, 2]):
+            b[:, off:off + 2] = np.full(b.shape[0], 0.001, dtype=np.float16).view(np.uint8).reshape(-1, 2)
+        b = b.reshape(-1)
+    else:
+        from candy_b200.backend import QStorage
+        b = QStorage.quantize(device, qt, order, (rng.standard_normal((n, k)) * 0.02).astype(np.float32)).data()
+    out = device.alloc(n * k)  # the library's dequantizer is bit-exact against the oracle's (its own tests)
+    src = device.upload_bytes(b)
+    per = 256 if qt in abi.K_BLOCK_BYTES else 32
+    abi.check(device.ctx, device._lib.cq_dequantize(device.ctx, qt, order, src.ptr, n * k // per, out.ptr), "dequantize")
+    return b, out.data().reshape(n, k).astype(np.float64)
+
+
+FORMATS = [(abi.Q4_0, 0), (abi.Q4_0, 1), (abi.Q8_0, 0), (abi.Q4_1, 0), (abi.Q4_1, 1), (abi.Q5_0, 1), (abi.Q5_1, 1), (abi.Q4_K, 1), (abi.Q5_K, 1), (abi.Q6_K, 1)]
+
+
+@pytest.mark.parametrize("qt,order", FORMATS)
+@pytest.mark.parametrize("m,n,k", [(1, 1, 32), (1, 5000, 1056), (2, 700, 4192), (3, 301, 96), (5, 9600, 480), (8, 3, 14560), (9, 130, 7200), (20, 2000, 1056)])
+def test_plain_f32(device, qt, order, m, n, k):
+    if qt in abi.K_BLOCK_BYTES:
+        k = (k + 255) // 256 * 256
+    if qt not in (abi.Q4_0, abi.Q8_0) and m == 1 and k % 256 == 0 and qt not in abi.K_BLOCK_BYTES:
+        pytest.skip("the streaming kernel's")
+    if qt not in (abi.Q4_0, abi.Q8_0) and m > 8:
+        m = 8
+    blocks, w = blocks_of(device, qt, order, n, k, m + n + k)
+    x = np.random.default_rng(m).standard_normal((m, k)).astype(np.float32)
+    bias = np.random.default_rng(n).standard_normal(n).astype(np.float32) if n > 1000 else None
+    y = run(device, qt, order, ACT_F32, blocks, n, x, k + 4, bias)
+    want = x.astype(np.float64) @ w.T
+    # f32 sums of the products, some thirty additions after one another per lane and block: 2^-24 each, of the sum of magnitudes
+    bound = 2.0 ** -24 * (k / 32 + 48) * (np.abs(x).astype(np.float64) @ np.abs(w).T) * 2
+    if bias is not None:
+        want, bound = want + bias, bound + 2.0 ** -22 * np.abs(bias)
+    if qt in (abi.Q4_1, abi.Q5_1, abi.Q4_K, abi.Q5_K):  # q * scale and the minimum are summed apart and cancel: magnitudes of both
+        bound = bound * 16
+    assert (np.abs(y - want) <= bound).all()
+
+
+@pytest.mark.parametrize("qt,order", [(abi.Q4_0, 0), (abi.Q8_0, 0), (abi.Q5_0, 1)])
+def test_plain_f32_at_odd_addresses(device, qt, order):
+    n, k, m = 300, 544, 3
+    blocks, w = blocks_of(device, qt, order, n, k, 1)
+    x = np.random.default_rng(2).standard_normal((m, k)).astype(np.float32)
+    y = run(device, qt, order, ACT_F32, blocks, n, x, w_off=2)
+    base = run(device, qt, order, ACT_F32, blocks, n, x)
+    assert (y == base).all()
+    assert np.abs(y - x.astype(np.float64) @ w.T).max() <= 1e-6 * np.abs(x.astype(np.float64) @ w.T).max() * 4
+    if qt != abi.Q5_0:  # x at 4-byte alignment, an odd row pitch
+        assert (run(device, qt, order, ACT_F32, blocks, n, x, k + 1, x_off=4) == base).all()
+
+
+@pytest.mark.parametrize("qt,order", [(abi.Q4_0, 0), (abi.Q4_0, 1), (abi.Q8_0, 0)])
+@pytest.mark.parametrize("m,n,k", [(1, 300, 32), (1, 4096, 4192), (2, 129, 480), (7, 1000, 1056), (9, 700, 288), (70, 300, 4192), (300, 257, 224)])
+@pytest.mark.parametrize("act", [ACT_Q8_1, ACT_F16])
+def test_padded_routes(device, qt, order, m, n, k, act):
+    blocks, w = blocks_of(device, qt, order, n, k, m + n + k)
+    x = np.random.default_rng(m).standard_normal((m, k)).astype(np.float32)
+    bias = np.random.default_rng(n).standard_normal(n).astype(np.float32) if n > 500 else None
+    y = run(device, qt, order, act, blocks, n, x, k + 3, bias, w_off=2, x_off=4)
+    if act == ACT_Q8_1:
+        want = oc.qmatmul(qt, order, x, blocks, n, nthreads=8, q8_1=True)
+    else:
+        want = x.astype(np.float16).astype(np.float64) @ w.astype(np.float16).astype(np.float64).T
+    if bias is not None:
+        want = want + bias
+    assert np.abs(y - want).max() <= 2e-5 * np.abs(want).max()
+
+
+def test_padded_route_in_a_capture(device):
+    """Captured without the room for the copies the call takes the plain route; captured after a first run it takes the copies."""
+    from candy_b200.backend import CudaDevice
+    dev = CudaDevice(0)
+    n, k, m = 256, 544, 9
+    blocks, _ = blocks_of(dev, abi.Q8_0, 0, n, k, 5)
+    x = np.random.default_rng(6).standard_normal((m, k)).astype(np.float32)
+    wb, xd, yd = dev.upload_bytes(blocks), dev.storage_from_slice(x), dev.zeros(m * n)
+    lib, ctx = dev._lib, dev.ctx
+    want = oc.qmatmul(abi.Q8_0, 0, x, blocks, n, nthreads=8, q8_1=True)
+    abi.check(ctx, lib.cq_reserve(ctx, 8 * (k // 32) * 36), "reserve")  # what the plain route needs for eight rows
+    for _ in range(2):
+        g = C.c_void_p()
+        abi.check(ctx, lib.cq_capture_begin(ctx), "begin")
+        abi.check(ctx, lib.cq_qmatmul(ctx, abi.Q8_0, 0, ACT_Q8_1, xd.ptr, m, k, k, wb.ptr, n, yd.ptr, n), "matmul")
+        abi.check(ctx, lib.cq_capture_end(ctx, C.byref(g)), "end")
+        abi.check(ctx, lib.cq_graph_launch(ctx, g), "launch")
+        dev.synchronize()
+        assert np.abs(yd.data().reshape(m, n) - want).max() <= 2e-5 * np.abs(want).max()
+        lib.cq_graph_destroy(ctx, g)
+        abi.check(ctx, lib.cq_qmatmul(ctx, abi.Q8_0, 0, ACT_Q8_1, xd.ptr, m, k, k, wb.ptr, n, yd.ptr, n), "first run")
+        abi.check(ctx, lib.cq_memset(ctx, yd.ptr, 0, 4 * m * n), "clear")
+        dev.synchronize()
+    dev.close()

@@ -87,6 +87,27 @@ cq_status cq_reserve_scratch(cq_ctx *ctx, size_t bytes) {
     return CQ_OK;
 }
 
+// Room for padded operands; false (and nothing done) where it would have to grow during capture, or the device is full.
+static bool reserve_pad(cq_ctx *ctx, size_t bytes) {
+    if (bytes <= ctx->pad_bytes) return true;
+    if (stream_capturing(ctx)) return false;
+    if (ctx->pad) {
+        if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) return false;
+        if (ctx->graphs_alive > 0) ctx->retired_scratch.push_back(ctx->pad);  // graphs may still point into it
+        else cudaFree(ctx->pad);
+        ctx->pad = nullptr;
+        ctx->pad_bytes = 0;
+    }
+    const size_t want = (bytes + 0xFFFFF) & ~size_t(0xFFFFF);
+    if (cq_device_malloc(ctx, &ctx->pad, want) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->pad = nullptr;
+        return false;
+    }
+    ctx->pad_bytes = want;
+    return true;
+}
+
 void cq_w16_invalidate(cq_ctx *ctx, const void *begin, size_t bytes) {
     if (ctx->w16_cache.empty() || !begin || bytes == 0) return;
     const uintptr_t lo = reinterpret_cast<uintptr_t>(begin), hi = lo + bytes;
@@ -174,6 +195,7 @@ cq_status cq_ctx_destroy(cq_ctx *ctx) {
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     if (ctx->scratch) cudaFree(ctx->scratch);
+    if (ctx->pad) cudaFree(ctx->pad);
     for (void *p : ctx->retired_scratch) cudaFree(p);
     for (auto &kv : ctx->w16_cache) cudaFree(kv.second);
     idle_release(ctx);
@@ -413,6 +435,33 @@ cq_status cq_qmatmul(cq_ctx *ctx, int qtype, int order, int actmode, const float
     CQ_ENTER(ctx);
     cq_status s = check_matmul_args(ctx, qtype, order, actmode, x_dev, m, k, ldx, w_blocks_dev, n, y_dev, ldy);
     if (s != CQ_OK) return s;
+    // Rows that are not multiples of 256 values (their blocks start at any even address, which no bulk or tensor copy takes):
+    // weights and activations are copied with zero blocks and zeros behind each row, and the copies take the fast routes.
+    // Without that these calls run one warp per weight row, eight rows of x at a time (CQ_ACT_Q8_1), or through an f16 copy of
+    // W (CQ_ACT_F16).  n 11008, k 4192, Q4_0, us, without / with: CQ_ACT_Q8_1 1 row 35 / 29, 8 rows 169 / 35, 64 rows 1353 / 71;
+    // CQ_ACT_F16 1 row 79 / 33, 64 rows 74 / 44, 128 rows 64 / 55, but 256 rows 67 / 72.  The copy costs about 20 us there, a
+    // launch and little else on a small matrix (1 row of 700 x 1056, Q8_1: 8.3 / 16), hence the lines.  CQ_ACT_F32 keeps its
+    // plain f32 arithmetic for such rows.  The copies are outputs of a kernel, so nothing behind it may start early and
+    // fetch them.
+    const int64_t weights = n * k;
+    const bool pad_wins = actmode == CQ_ACT_Q8_1 ? m >= 9 || weights >= (m == 1 ? int64_t(24) << 20 : int64_t(8) << 20)
+                                                 : actmode == CQ_ACT_F16 && (m <= 8 || (m <= 128 && weights >= int64_t(8) << 20));
+    if (k % 256 != 0 && (qtype == CQ_Q4_0 || qtype == CQ_Q8_0) && pad_wins && !(actmode == CQ_ACT_F16 && (ctx->tune.gemm_cache_weights || ctx->tune.gemm_variant != 0)) &&
+        !ctx->tune.force_simple && !ctx->fuse.on && ctx->push.world == 0 && ctx->tune.gemm_int8 && n <= (1 << 27) &&
+        (reinterpret_cast<uintptr_t>(w_blocks_dev) & 1) == 0 && (reinterpret_cast<uintptr_t>(x_dev) & 3) == 0 && (reinterpret_cast<uintptr_t>(y_dev) & 3) == 0) {
+        const int64_t kp = (k + 255) / 256 * 256;
+        const size_t wb = (cq_blocks_bytes(qtype, n, kp) + 255) & ~size_t(255);
+        if (reserve_pad(ctx, wb + (size_t)m * kp * sizeof(float))) {
+            float *xp = reinterpret_cast<float *>(static_cast<uint8_t *>(ctx->pad) + wb);
+            s = launch_pad_rows(ctx, qtype, w_blocks_dev, n, ctx->pad, x_dev, m, k, ldx, xp, kp);
+            if (s != CQ_OK) return s;
+            const int pdl = ctx->tune.pdl;
+            ctx->tune.pdl = 0;
+            s = cq_qmatmul(ctx, qtype, order, actmode, xp, m, kp, kp, ctx->pad, n, y_dev, ldy);
+            ctx->tune.pdl = pdl;
+            if (s == CQ_OK || !stream_capturing(ctx)) return s;  // (capturing without the scratch for that: the plain route below)
+        }
+    }
     // Two to eight rows against Q4_0 in CQ_ACT_F32 or CQ_ACT_Q8_1: the streaming kernel with tensor-core block dots, one launch
     // (two rows only against large weights, or in CQ_ACT_Q8_1 long rows: elsewhere the two-row form of the one-row kernel is quicker)
     if (actmode != CQ_ACT_F16 && ctx->tune.gemv_mma > 0 && (m >= ctx->tune.gemv_mma || (m == 2 && (actmode == CQ_ACT_Q8_1 ? (k >= 8192 || n * k >= (int64_t(100) << 20)) : n * k >= (int64_t(40) << 20)))) && m <= 8 &&

@@ -89,6 +89,8 @@ struct cq_ctx {
     int *dev_err_devptr = nullptr;
     void *scratch = nullptr;      // activation staging (Q8_1 blocks / f16 copies)
     size_t scratch_bytes = 0;
+    void *pad = nullptr;          // weights and activations with rows padded to whole chunks of 256 values (see cq_qmatmul)
+    size_t pad_bytes = 0;
     std::vector<void *> retired_scratch;  // outgrown blocks that instantiated graphs may still reference
     int graphs_alive = 0;                 // graphs made by cq_capture_end and not yet destroyed
     void *xfer_x = nullptr;       // device staging used by cq_qmatmul_host
@@ -141,6 +143,8 @@ void cq_w16_invalidate(cq_ctx *ctx, const void *begin, size_t bytes);
 // ---- launchers implemented in the kernel translation units -------------------------
 cq_status launch_dequantize(cq_ctx *ctx, int qtype, int order, const void *blocks, int64_t nblocks, float *y);
 cq_status launch_quantize_rows(cq_ctx *ctx, int qtype, int order, const float *w, int64_t nblocks, void *blocks);
+cq_status launch_pad_rows(cq_ctx *ctx, int qtype, const void *w, int64_t n, void *w_out, const float *x, int64_t m, int64_t k, int64_t ldx, float *x_out,
+                          int64_t k_out);
 cq_status launch_quantize_q8_1(cq_ctx *ctx, const float *x, int64_t m, int64_t k, int64_t ldx, void *out);
 cq_status launch_gemv(cq_ctx *ctx, int qtype, int order, int actmode, const float *x, int64_t m, int64_t k,
                       int64_t ldx, const void *w, int64_t n, float *y, int64_t ldy);

@@ -195,7 +195,53 @@ __global__ void __launch_bounds__(256) quantize_q8_1_kernel(const float *__restr
     }
 }
 
+// Rows of blocks and rows of x copied with their length rounded up: zero blocks and zero values follow the last ones.
+// A warp per row, 16 bytes per lane and trip: source rows start at any even address, so a lane reads the five aligned words
+// around its 16 bytes and shifts them into place.  A word that only touches a row's end lies within four bytes that hold a byte of the row.
+constexpr int kPadWarps = 8;
+__global__ void __launch_bounds__(32 * kPadWarps) pad_rows_kernel(const uint8_t *__restrict__ w, int64_t n, int row_bytes, int row_out,
+                                                                uint8_t *__restrict__ w_out, const float *__restrict__ x, int64_t m, int k, int64_t ldx,
+                                                                float *__restrict__ x_out, int k_out) {
+    const int lane = threadIdx.x & 31;
+    const int64_t row = (int64_t)blockIdx.x * kPadWarps + (threadIdx.x >> 5);
+    if (row < n) {
+        const uint8_t *src = w + row * row_bytes;
+        const uint32_t odd = (uint32_t)(reinterpret_cast<uintptr_t>(src) & 2);
+        const uint8_t *base = src - odd;
+        uint4 *dst = reinterpret_cast<uint4 *>(w_out + row * row_out);
+#pragma unroll 4
+        for (int c = lane; c < row_out / 16; c += 32) {
+            uint32_t v[5], o[4];
+#pragma unroll
+            for (int i = 0; i < 5; ++i) {
+                const int at = 16 * c + 4 * i;  // this word holds bytes at - odd .. at - odd + 3 of the row
+                v[i] = at - (int)odd < row_bytes && (i < 4 || odd) ? __ldg(reinterpret_cast<const uint32_t *>(base + at)) : 0u;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int at = 16 * c + 4 * i;
+                o[i] = __funnelshift_r(v[i], v[i + 1], 8 * odd);
+                if (at + 4 > row_bytes) o[i] = at + 2 == row_bytes ? o[i] & 0xFFFFu : (at >= row_bytes ? 0u : o[i]);
+            }
+            dst[c] = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+    } else if (row < n + m) {
+        const float *src = x + (row - n) * ldx;
+        float *dst = x_out + (row - n) * k_out;
+        for (int i = lane; i < k_out; i += 32) dst[i] = i < k ? src[i] : 0.0f;
+    }
+}
+
 }  // namespace
+
+cq_status launch_pad_rows(cq_ctx *ctx, int qtype, const void *w, int64_t n, void *w_out, const float *x, int64_t m, int64_t k, int64_t ldx, float *x_out,
+                          int64_t k_out) {
+    const int bb = qtype == CQ_Q4_0 ? kQ4Bytes : kQ8Bytes;
+    pad_rows_kernel<<<(unsigned)((n + m + kPadWarps - 1) / kPadWarps), 32 * kPadWarps, 0, ctx->stream>>>(
+        static_cast<const uint8_t *>(w), n, (int)(k / kQK) * bb, (int)(k_out / kQK) * bb, static_cast<uint8_t *>(w_out), x, m, (int)k, ldx, x_out, (int)k_out);
+    CQ_CUDA(ctx, cudaGetLastError());
+    return CQ_OK;
+}
 
 cq_status launch_dequantize(cq_ctx *ctx, int qtype, int order, const void *blocks, int64_t nblocks, float *y) {
     const bool vec = (reinterpret_cast<uintptr_t>(y) & 15) == 0;

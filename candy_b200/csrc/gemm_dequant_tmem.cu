@@ -23,8 +23,8 @@
 //                 is multiplied.
 //   1 lane/pipe   issues tcgen05.mma (A from tensor memory, B = X slab through a shared-memory
 //                 descriptor), M=128, N=MPAD, K=16, sixteen per item, into the pipe's own f32
-//                 accumulator.  A single thread can start an MMA only every ~90 cycles whatever
-//                 its shape -- far too slow for narrow N -- hence one issuer per pipe.
+//                 accumulator.  A lane that runs the issuing loop alone starts an MMA only every ~90
+//                 cycles whatever its shape; the issuing warps run it as a whole, see there.
 //   4 warps       epilogue: tcgen05.ld, store.  Lane = weight row, so for each batch row a warp
 //                 writes 32 consecutive floats.
 //
@@ -107,16 +107,16 @@ __global__ void __launch_bounds__(256) x_to_f16_perm_kernel(const float *__restr
 
 // Groups of tiles whose k range was shared between CTAs: y[m][j] = sum of the CTAs' partials, in
 // CTA order.  CTA i owns steps [i*per_cta, (i+1)*per_cta); a group's steps are [t*nchunks, (t+1)*nchunks).
-// One block per (group, batch row), one thread per four columns.
-__global__ void __launch_bounds__(64) shared_group_sum_kernel(const float *__restrict__ part, int64_t m, int64_t n, int nchunks, int per_cta,
+// One block per (group, four batch rows), one thread per four columns.
+__global__ void __launch_bounds__(256) shared_group_sum_kernel(const float *__restrict__ part, int64_t m, int64_t n, int nchunks, int per_cta,
                                                             float *__restrict__ y, int64_t ldy) {
     constexpr int kGroupRows = 256;
     pdl_launch_dependents();
     pdl_wait_prior();
-    const int t = blockIdx.x, row = blockIdx.y;
+    const int t = blockIdx.x, row = blockIdx.y * 4 + (threadIdx.x >> 6);
     const int first = (t * nchunks) / per_cta, last = ((t + 1) * nchunks - 1) / per_cta;
-    if (first == last) return;  // one CTA had the group's whole k range and wrote y itself
-    const int r = threadIdx.x * 4;
+    if (first == last || row >= m) return;  // one CTA had the group's whole k range and wrote y itself
+    const int r = (threadIdx.x & 63) * 4;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int c = first; c <= last; ++c) {
         const int slot = 2 * c + (((c * per_cta) / nchunks == t) ? 0 : 1);
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(FtCfg<QT, MPAD>::kThreads, 1)
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(d_empty + 1);
     uint32_t *sink = tmem_slot + 1;  // one word per warp: target of the stores that pin load completion (see the dequantizing warps)
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     // Chained launch: the next kernel may become resident now.  Here, only the warps that touch what
     // earlier kernels produce or still read wait for them: the X loaders (X scratch) and the epilogue
     // (y, partial sums).  The raw blocks are nobody's output, so their TMA warps start at once.
@@ -303,8 +303,9 @@ __global__ void __launch_bounds__(FtCfg<QT, MPAD>::kThreads, 1)
                     }
         }
     } else if (warp < Cfg::kWarpDq0) {
-        // ---- MMA: issuer (pipe q, parity e) takes every second K=16 step of both halves ----------------
-        if (lane == 0) {
+        // ---- MMA: issuer (pipe q, parity e) takes every second K=16 step of both halves; the whole warp runs the loop, so
+        // that descriptors stay in uniform registers, and one lane issues (57344 x 8192 Q4_0, 32 rows: 85 -> 73 us a call) ----
+        {
             constexpr uint32_t idesc = idesc_f16(FT_ROWS, MPAD);
             const int iss = warp - Cfg::kWarpMma0, q = iss / IPP, e = iss % IPP;
             int step = 0, seg = 0;
@@ -314,41 +315,40 @@ __global__ void __launch_bounds__(FtCfg<QT, MPAD>::kThreads, 1)
                 int group, c0, cn;
                 segment(g, group, c0, cn);
                 g += cn;
-                if (seg >= 1 && !mbar_wait_sleep(smem_u32(&d_empty[0]), (seg - 1) & 1, 100)) {  // epilogue has read the accumulators
-                    atomicExch(p.err, kDevErrMma);
+                if (seg >= 1 && !__all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&d_empty[0]), (seg - 1) & 1))) {  // epilogue has read the accumulators
+                    if (lane == 0) atomicExch(p.err, kDevErrMma);
                     break;
                 }
                 tc_fence_after();
                 for (int c = 0; c < cn && ok; ++c, ++step) {
                     const int xs = step % XST;
-                    if (!mbar_wait_sleep(smem_u32(&x_full[xs]), (step / XST) & 1, 40)) {
-                        atomicExch(p.err, kDevErrFullWait);
-                        ok = false;
-                        break;
-                    }
                     const uint64_t bdesc = smem_desc_k128(smem_u32(smem_x + (size_t)xs * Cfg::kXBytes));
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
-                        if (!mbar_wait_sleep(smem_u32(&a_full[2 * q + h]), step & 1, 20)) {
-                            atomicExch(p.err, kDevErrFullWait);
+                        const bool there = (h || mbar_wait_bounded(smem_u32(&x_full[xs]), (step / XST) & 1)) && mbar_wait_bounded(smem_u32(&a_full[2 * q + h]), step & 1);
+                        if (!__all_sync(0xffffffffu, there)) {
+                            if (lane == 0) atomicExch(p.err, kDevErrFullWait);
                             ok = false;
                             break;
                         }
                         tc_fence_after();
                         const uint32_t a_t = tmem_base + (uint32_t)(q * FT_ACOLS + h * 64);
-                        {
+                        if (elect_one()) {
 #pragma unroll
                             for (int j2 = 0; j2 < 8 / IPP; ++j2) {
                                 const int j = IPP * j2 + e;  // K=16 step inside the half
                                 const int jj = 8 * h + j;  // ... inside the item: X box jj/4, 32-byte column jj%4
                                 tc_mma_f16_ts(acc, a_t + 8 * j, bdesc + (uint64_t)((jj >> 2) * (MPAD * 128 / 16) + (jj & 3) * 2), idesc, (c | h | j2) != 0);
                             }
+                            tc_commit(smem_u32(&a_empty[2 * q + h]));
+                            if (h == 1) {
+                                tc_commit(smem_u32(&x_empty[xs]));
+                                if (c == cn - 1) tc_commit(smem_u32(&d_full[0]));
+                            }
                         }
-                        tc_commit(smem_u32(&a_empty[2 * q + h]));
+                        __syncwarp();
                     }
-                    tc_commit(smem_u32(&x_empty[xs]));
                 }
-                tc_commit(smem_u32(&d_full[0]));
             }
         }
     } else if (warp < Cfg::kWarpEp0) {
@@ -590,7 +590,7 @@ cq_status launch_qgemm_dequant_tmem(cq_ctx *ctx, int qtype, int order, const flo
     if (s != CQ_OK) return s;
     if (shared_tiles) {
         static_assert(FtCfg<CQ_Q4_0, 16>::kGroupRows == 256 && FtCfg<CQ_Q8_0, 64>::kGroupRows == 256 && FtCfg<CQ_Q4_0, 128>::kGroupRows == 256, "sum kernel layout");
-        s = launch_chained(ctx, shared_group_sum_kernel, dim3((unsigned)ngroups, (unsigned)m), dim3(64), 0, (const float *)part, m, n, nchunks, (int)per_cta, y, ldy);
+        s = launch_chained(ctx, shared_group_sum_kernel, dim3((unsigned)ngroups, (unsigned)((m + 3) / 4)), dim3(256), 0, (const float *)part, m, n, nchunks, (int)per_cta, y, ldy);
         if (s != CQ_OK) return s;
     }
     return CQ_OK;

@@ -38,33 +38,57 @@ struct GemmCfg {
 };
 
 // ---- f16 conversion kernels -------------------------------------------------------------
-__global__ void __launch_bounds__(256) x_to_f16_kernel(const float *__restrict__ x, int64_t m, int64_t k, int64_t ldx,
-                                                     __half *__restrict__ out) {
+// CTA `cta` of `ctas` of X [m, k] f32 -> f16: 16 bytes in where X allows it.
+__device__ __forceinline__ void x_part_to_f16(const float *__restrict__ x, int64_t m, int64_t k, int64_t ldx, __half *__restrict__ out, unsigned cta,
+                                              unsigned ctas) {
     const int64_t total = m * (k / 4);
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+    const bool vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0 && ldx % 4 == 0;
+    for (int64_t i = (int64_t)cta * blockDim.x + threadIdx.x; i < total; i += (int64_t)ctas * blockDim.x) {
         const int64_t row = i / (k / 4), c4 = i - row * (k / 4);
         const float *src = x + row * ldx + c4 * 4;
-        __half2 a = __floats2half2_rn(src[0], src[1]), b = __floats2half2_rn(src[2], src[3]);
+        const float4 t = vec ? *reinterpret_cast<const float4 *>(src) : make_float4(src[0], src[1], src[2], src[3]);
+        __half2 a = __floats2half2_rn(t.x, t.y), b = __floats2half2_rn(t.z, t.w);
         uint2 v;
         v.x = *reinterpret_cast<uint32_t *>(&a);
         v.y = *reinterpret_cast<uint32_t *>(&b);
         *reinterpret_cast<uint2 *>(out + row * k + c4 * 4) = v;
     }
 }
+__global__ void __launch_bounds__(256) x_to_f16_kernel(const float *__restrict__ x, int64_t m, int64_t k, int64_t ldx, __half *__restrict__ out) {
+    x_part_to_f16(x, m, k, ldx, out, blockIdx.x, gridDim.x);
+}
 
-// One thread converts 8 consecutive values of a block (one 16-byte store).  The f32 value
+// Eight bytes that start at any even address, as two words: the aligned words around them, shifted into place.
+__device__ __forceinline__ void eight_bytes(const uint8_t *p, uint32_t &a, uint32_t &b) {
+    const uint32_t odd = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 2);
+    const uint32_t *q = reinterpret_cast<const uint32_t *>(p - odd);
+    const uint32_t v0 = q[0], v1 = q[1], v2 = odd ? q[2] : 0u;
+    a = __funnelshift_r(v0, v1, 8 * odd);
+    b = __funnelshift_r(v1, v2, 8 * odd);
+}
+
+// Both f16 copies in one launch: the first x_ctas CTAs convert X, the others W.
+// W: one thread converts 8 consecutive values of a block (one 16-byte store).  The f32 value
 // d*(q-8) (or d*q) is exact, so the only rounding is f32 -> f16, round-to-nearest-even.
+// Bound: HBM (0.56 / 1.06 bytes in, 2 out per weight).  One launch that the GEMM may overlap instead of two that it may
+// not: n 11008, k 4096, 2048 rows of Q8_0 183 -> 172 us a call, of Q4_0 in the split order 183 -> 170.
 template <int QT, int ORDER>
-__global__ void __launch_bounds__(256) w_to_f16_kernel(const uint8_t *__restrict__ blocks, int64_t nblocks,
-                                                     __half *__restrict__ out) {
+__global__ void __launch_bounds__(256) operands_to_f16_kernel(const uint8_t *__restrict__ blocks, int64_t nblocks, __half *__restrict__ out, unsigned x_ctas,
+                                                            const float *__restrict__ x, int64_t m, int64_t k, int64_t ldx, __half *__restrict__ x_out) {
+    pdl_launch_dependents();  // the GEMM sets itself up meanwhile
+    if (blockIdx.x < x_ctas) {
+        x_part_to_f16(x, m, k, ldx, x_out, blockIdx.x, x_ctas);
+        return;
+    }
     const int64_t total = nblocks * 4;
-    for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t step = (int64_t)(gridDim.x - x_ctas) * blockDim.x;
+    for (int64_t idx = (int64_t)(blockIdx.x - x_ctas) * blockDim.x + threadIdx.x; idx < total; idx += step) {
         const int64_t blk = idx >> 2;
         const int p = (int)(idx & 3);  // values 8p .. 8p+7
         float v[8];
+        const uint8_t *b = blocks + blk * (QT == CQ_Q4_0 ? kQ4Bytes : kQ8Bytes);
+        const float d = __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(b)));
         if (QT == CQ_Q4_0) {
-            const uint8_t *b = blocks + blk * kQ4Bytes;
-            const float d = __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(b)));
             if (ORDER == CQ_ORDER_GO_INTERLEAVED) {
                 const uint8_t *qs = b + 2 + 4 * p;  // bytes 4p..4p+3 -> values 8p..8p+7
                 const uint32_t four = *reinterpret_cast<const unsigned short *>(qs) |
@@ -72,16 +96,17 @@ __global__ void __launch_bounds__(256) w_to_f16_kernel(const uint8_t *__restrict
 #pragma unroll
                 for (int i = 0; i < 8; ++i) v[i] = d * (float)((int)((four >> (4 * i)) & 0xF) - 8);
             } else {
-                const uint8_t *qs = b + 2 + 8 * (p & 1);  // values 8p..8p+7 = low (p<2) or high nibbles of 8 bytes
+                uint32_t w[2];  // values 8p .. = low (p < 2) or high nibbles of 8 bytes
+                eight_bytes(b + 2 + 8 * (p & 1), w[0], w[1]);
                 const int sh = (p >= 2) ? 4 : 0;
 #pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] = d * (float)((int)((qs[i] >> sh) & 0xF) - 8);
+                for (int i = 0; i < 8; ++i) v[i] = d * (float)((int)((w[i >> 2] >> (8 * (i & 3) + sh)) & 0xF) - 8);
             }
         } else {
-            const uint8_t *b = blocks + blk * kQ8Bytes;
-            const float d = __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(b)));
+            uint32_t w[2];
+            eight_bytes(b + 2 + 8 * p, w[0], w[1]);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = d * (float)(int)(signed char)b[2 + 8 * p + i];
+            for (int i = 0; i < 8; ++i) v[i] = d * (float)(int)(signed char)((w[i >> 2] >> (8 * (i & 3))) & 0xFF);
         }
         __half2 h[4];
 #pragma unroll
@@ -103,7 +128,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     uint64_t *full = bars, *empty = bars + STAGES, *acc_full = bars + 2 * STAGES;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     // m-tiles vary fastest across the grid: a wave of CTAs then shares a handful of B tiles (and all
     // of A), so the f16 weight copy crosses HBM about once instead of once per few m-tiles.
     const int tile_m = blockIdx.x, tile_n = blockIdx.y;
@@ -147,24 +172,25 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                 }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {  // the whole warp runs the loop, one lane issues (n 11008, k 4096, 64 rows of Q4_1: 77 -> 66 us a call)
             constexpr uint32_t idesc = idesc_f16(BM, BN);
-            bool ok = true;
-            for (int kb = 0; kb < nk && ok; ++kb) {
+            for (int kb = 0; kb < nk; ++kb) {
                 const int s = kb % STAGES;
-                if (!mbar_wait_bounded(smem_u32(&full[s]), (kb / STAGES) & 1)) {
-                    atomicExch(err, kDevErrFullWait);
-                    ok = false;
+                if (!__all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&full[s]), (kb / STAGES) & 1))) {
+                    if (lane == 0) atomicExch(err, kDevErrFullWait);
                     break;
                 }
                 tc_fence_after();
                 const uint32_t a0 = smem_u32(smA + (size_t)s * A_BYTES), b0 = smem_u32(smB + (size_t)s * B_BYTES);
+                if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < BK / 16; ++k)  // 16 values of k = 32 bytes inside the 128-byte swizzled row
-                    tc_mma_f16(tmem_base, smem_desc_k128(a0 + 32 * k), smem_desc_k128(b0 + 32 * k), idesc, (kb | k) != 0);
-                tc_commit(smem_u32(&empty[s]));  // arrives when these MMAs have finished reading the stage
+                    for (int k = 0; k < BK / 16; ++k)  // 16 values of k = 32 bytes inside the 128-byte swizzled row
+                        tc_mma_f16(tmem_base, smem_desc_k128(a0 + 32 * k), smem_desc_k128(b0 + 32 * k), idesc, (kb | k) != 0);
+                    tc_commit(smem_u32(&empty[s]));  // arrives when these MMAs have finished reading the stage
+                }
+                __syncwarp();
             }
-            tc_commit(smem_u32(acc_full));  // arrives when every MMA issued so far has completed
+            if (elect_one()) tc_commit(smem_u32(acc_full));  // arrives when every MMA issued so far has completed
         }
     } else {
         // epilogue warps 2..5: warp w may touch TMEM lanes 32*(w%4) .. +31 only
@@ -399,6 +425,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 
     if (warp == 0) {
         if (lane == 0) {
+            pdl_wait_prior();  // the f16 copies come from the kernel before
             int it = 0;
             bool ok = true;
             for (int t = pair; t < ntiles && ok; t += npairs) {
@@ -577,25 +604,24 @@ cq_status launch_gemm(cq_ctx *ctx, int qtype, int order, int actmode, const floa
     __half *x16 = static_cast<__half *>(ctx->scratch);
     if (!w16) w16 = reinterpret_cast<__half *>(static_cast<uint8_t *>(ctx->scratch) + x16_bytes);
     const unsigned cap = (unsigned)ctx->sm_count * 16;
-    {
-        const int64_t total = m * (k / 4);
-        const unsigned grid = (unsigned)((total + 255) / 256 < cap ? (total + 255) / 256 : cap);
-        x_to_f16_kernel<<<grid, 256, 0, ctx->stream>>>(x, m, k, ldx, x16);
-    }
-    if (need_convert) {
+    const int64_t xtotal = m * (k / 4);
+    const unsigned xgrid = (unsigned)((xtotal + 255) / 256 < cap ? (xtotal + 255) / 256 : cap);
+    bool chained = false;  // the kernel before the GEMM lets it start early
+    if (need_convert && (qtype == CQ_Q4_0 || qtype == CQ_Q8_0)) {
         const int64_t nblocks = n * (k / kQK);
         const int64_t total = nblocks * 4;
-        const unsigned grid = (unsigned)((total + 255) / 256 < cap ? (total + 255) / 256 : cap);
+        const unsigned grid = xgrid + (unsigned)((total + 255) / 256 < cap ? (total + 255) / 256 : cap);
         const uint8_t *wb = static_cast<const uint8_t *>(w);
-        if (cq_is_k_format(qtype)) {
-            cq_status s2 = launch_w_to_f16_k(ctx, qtype, w, n * (k / 256), w16);
+        if (qtype == CQ_Q4_0 && order == CQ_ORDER_GO_INTERLEAVED) operands_to_f16_kernel<CQ_Q4_0, 0><<<grid, 256, 0, ctx->stream>>>(wb, nblocks, w16, xgrid, x, m, k, ldx, x16);
+        else if (qtype == CQ_Q4_0) operands_to_f16_kernel<CQ_Q4_0, 1><<<grid, 256, 0, ctx->stream>>>(wb, nblocks, w16, xgrid, x, m, k, ldx, x16);
+        else operands_to_f16_kernel<CQ_Q8_0, 0><<<grid, 256, 0, ctx->stream>>>(wb, nblocks, w16, xgrid, x, m, k, ldx, x16);
+        chained = true;
+    } else {
+        x_to_f16_kernel<<<xgrid, 256, 0, ctx->stream>>>(x, m, k, ldx, x16);
+        if (need_convert) {
+            cq_status s2 = cq_is_k_format(qtype) ? launch_w_to_f16_k(ctx, qtype, w, n * (k / 256), w16) : launch_w_to_f16_more(ctx, qtype, order, w, n * (k / kQK), w16);
             if (s2 != CQ_OK) return s2;
-        } else if (cq_is_more_format(qtype)) {
-            cq_status s2 = launch_w_to_f16_more(ctx, qtype, order, w, nblocks, w16);
-            if (s2 != CQ_OK) return s2;
-        } else if (qtype == CQ_Q4_0 && order == CQ_ORDER_GO_INTERLEAVED) w_to_f16_kernel<CQ_Q4_0, 0><<<grid, 256, 0, ctx->stream>>>(wb, nblocks, w16);
-        else if (qtype == CQ_Q4_0) w_to_f16_kernel<CQ_Q4_0, 1><<<grid, 256, 0, ctx->stream>>>(wb, nblocks, w16);
-        else w_to_f16_kernel<CQ_Q8_0, 0><<<grid, 256, 0, ctx->stream>>>(wb, nblocks, w16);
+        }
     }
     CQ_CUDA(ctx, cudaGetLastError());
     CUtensorMap tmA, tmB;
@@ -616,9 +642,11 @@ cq_status launch_gemm(cq_ctx *ctx, int qtype, int order, int actmode, const floa
         static thread_local int configured_pair = -1;
         static thread_local int max_clusters = 0;
         cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
+        cudaLaunchAttribute attr[2];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = 2, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr, cfg.numAttrs = 1;
         cfg.blockDim = dim3(GEMM_THREADS);
         cfg.dynamicSmemBytes = P2_SMEM;
@@ -635,6 +663,7 @@ cq_status launch_gemm(cq_ctx *ctx, int qtype, int order, int actmode, const floa
             const int64_t ntiles = ((m + 255) / 256) * ((n + 255) / 256);
             const int64_t pairs = ntiles < max_clusters ? ntiles : max_clusters;
             cfg.gridDim = dim3((unsigned)(2 * pairs));
+            if (chained && ctx->tune.pdl) cfg.numAttrs = 2;
             CQ_CUDA(ctx, cudaLaunchKernelEx(&cfg, gemm_f16_tn_pair_kernel, tmA, tmBh, y, (int)m, (int)n, (int)k, ldy, ctx->dev_err_devptr));
             return CQ_OK;
         }

@@ -294,6 +294,22 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
     return d;
 }
 
+// Eight values of x in the order in which a dequantizing thread emits a word's weights, for 16-byte piece c (0..3) of a
+// 32-block: order 0 interleaved blocks, pairs (0,4) (1,5) (2,6) (3,7) of values 8c ..; order 1 split blocks, (0,2) (16,18)
+// (1,3) (17,19) of values 4c ..; order 2 as they lie.
+__device__ __forceinline__ void load_permuted8(const float *block, int c, int order, bool vec, float (&v)[8]) {
+    const float *p = block + (order == 1 ? 4 * c : 8 * c), *q = order == 1 ? p + 16 : p + 4;
+    float4 a, b;
+    if (vec) {
+        a = *reinterpret_cast<const float4 *>(p), b = *reinterpret_cast<const float4 *>(q);
+    } else {
+        a = make_float4(p[0], p[1], p[2], p[3]), b = make_float4(q[0], q[1], q[2], q[3]);
+    }
+    if (order == 0) v[0] = a.x, v[1] = b.x, v[2] = a.y, v[3] = b.y, v[4] = a.z, v[5] = b.z, v[6] = a.w, v[7] = b.w;
+    else if (order == 1) v[0] = a.x, v[1] = a.z, v[2] = b.x, v[3] = b.z, v[4] = a.y, v[5] = a.w, v[6] = b.y, v[7] = b.w;
+    else v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+}
+
 __device__ __forceinline__ void pdl_wait_prior() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 #endif  // __CUDACC__

@@ -77,28 +77,21 @@ struct FtCfg {
     static_assert(kDCol0 + kIssuers * kPipes * MPAD <= 512, "tensor memory");
 };
 
-// Position p of a block's 32 values, in the order the dequantizing threads emit them, holds
-// original element kPerm[order][p].
-__constant__ uint8_t kPerm[3][32] = {
-    {0, 4, 1, 5, 2, 6, 3, 7, 8, 12, 9, 13, 10, 14, 11, 15, 16, 20, 17, 21, 18, 22, 19, 23, 24, 28, 25, 29, 26, 30, 27, 31},
-    {0, 2, 16, 18, 1, 3, 17, 19, 4, 6, 20, 22, 5, 7, 21, 23, 8, 10, 24, 26, 9, 11, 25, 27, 12, 14, 28, 30, 13, 15, 29, 31},
-    // Q8_0: bytes convert in place, natural order
-    {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 17, 18, 19, 20, 21, 22, 23, 24, 25, 26, 27, 28, 29, 30, 31}};
-
 // X [m,k] f32 -> f16 with each 32-group permuted; one thread per eight output positions.
 __global__ void __launch_bounds__(256) x_to_f16_perm_kernel(const float *__restrict__ x, int64_t m, int64_t k, int64_t ldx, int order,
                                                           __half *__restrict__ out) {
     pdl_launch_dependents();  // the GEMM behind this kernel starts fetching weights meanwhile
     pdl_wait_prior();         // x comes from the previous kernel; the scratch this writes may still be read by it
     const int64_t per_row = k / 8, total = m * per_row;
+    const bool vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0 && ldx % 4 == 0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t row = i / per_row, o8 = i - row * per_row;  // output positions 8*o8 .. 8*o8+7 of the row
-        const float *src = x + row * ldx + (o8 >> 2) * 32;
-        const uint8_t *perm = kPerm[order] + (o8 & 3) * 8;
+        float v[8];
+        load_permuted8(x + row * ldx + (o8 >> 2) * 32, (int)(o8 & 3), order, vec, v);
         uint32_t w[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const __half2 h = __floats2half2_rn(src[perm[2 * j]], src[perm[2 * j + 1]]);
+            const __half2 h = __floats2half2_rn(v[2 * j], v[2 * j + 1]);
             w[j] = *reinterpret_cast<const uint32_t *>(&h);
         }
         *reinterpret_cast<uint4 *>(out + row * k + o8 * 8) = make_uint4(w[0], w[1], w[2], w[3]);

@@ -7,9 +7,9 @@
 //                  multiply-add away from hi); an activation, scaled by a power of two per row so that the row's largest
 //                  value sits just below 2^15, keeps 22 bits.  y = Xhi Whi + (Xlo Whi + Xhi Wlo); the dropped Xlo Wlo is
 //                  2^-22 of the product.  The bracket has an accumulator of its own: the tensor core truncates when it
-//                  adds, and small terms added to a large sum would each cost a truncation.  Measured against f64:
-//                  3e-6 (k = 4096) .. 2e-5 (k = 14336), where 15-bit block fixed point, which served these calls
-//                  before, shows 4.1e-5 at every k.
+//                  adds, and small terms added to a large sum would each cost a truncation.  Measured against f64
+//                  (2-norm): 1.2e-6 .. 4.7e-6 at k = 4096 .. 14336, where 15-bit block fixed point, which served these
+//                  calls before, shows 4.1e-5.
 //
 // What bounds it: the tensor pipe for large batches (three products per term in SPLIT), the weight stream for small ones.
 // The integer kernel that served CQ_ACT_F32 batches before has to scale every 32-term dot on the CUDA cores and stood at
@@ -76,27 +76,23 @@ struct GpParams {
     int *err;
 };
 
-// Position p of a block's 32 values, in the order the dequantizing threads emit them, holds original element
-// kGpPerm[order][p] (a dot product does not care; the activations are written in the same order).
-__constant__ uint8_t kGpPerm[3][32] = {
-    {0, 4, 1, 5, 2, 6, 3, 7, 8, 12, 9, 13, 10, 14, 11, 15, 16, 20, 17, 21, 18, 22, 19, 23, 24, 28, 25, 29, 26, 30, 27, 31},
-    {0, 2, 16, 18, 1, 3, 17, 19, 4, 6, 20, 22, 5, 7, 21, 23, 8, 10, 24, 26, 9, 11, 25, 27, 12, 14, 28, 30, 13, 15, 29, 31},
-    {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 17, 18, 19, 20, 21, 22, 23, 24, 25, 26, 27, 28, 29, 30, 31}};
-
 // ---- activation pre-passes ---------------------------------------------------------------------------------
+// Two 16-byte loads per eight values (value by value through a table of positions in constant memory: 128 rows x 4096 x 4096
+// 16.9 us a call instead of 16.2, CQ_ACT_F32 128 x 4096 x 11008 48.7 instead of 45.7).
 __global__ void __launch_bounds__(256) gp_x_f16_kernel(const float *__restrict__ x, int64_t m, int64_t k, int64_t ldx, int order,
                                                      __half *__restrict__ out) {
     pdl_launch_dependents();
     pdl_wait_prior();
     const int64_t per_row = k / 8, total = m * per_row;
+    const bool vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0 && ldx % 4 == 0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t row = i / per_row, o8 = i - row * per_row;
-        const float *src = x + row * ldx + (o8 >> 2) * 32;
-        const uint8_t *perm = kGpPerm[order] + (o8 & 3) * 8;
+        float v[8];
+        load_permuted8(x + row * ldx + (o8 >> 2) * 32, (int)(o8 & 3), order, vec, v);
         uint32_t w[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const __half2 h = __floats2half2_rn(src[perm[2 * j]], src[perm[2 * j + 1]]);
+            const __half2 h = __floats2half2_rn(v[2 * j], v[2 * j + 1]);
             w[j] = *reinterpret_cast<const uint32_t *>(&h);
         }
         *reinterpret_cast<uint4 *>(out + row * k + o8 * 8) = make_uint4(w[0], w[1], w[2], w[3]);
@@ -112,8 +108,16 @@ __global__ void __launch_bounds__(256) gp_x_split_kernel(const float *__restrict
     __shared__ float red[8];
     const int64_t row = blockIdx.x;
     const float *src = x + row * ldx;
+    const bool vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0 && ldx % 4 == 0;
     float amax = 0.0f;
-    for (int64_t i = threadIdx.x; i < k; i += 256) amax = fmaxf(amax, fabsf(src[i]));
+    if (vec) {
+        for (int64_t i = threadIdx.x; i < k / 4; i += 256) {
+            const float4 t = reinterpret_cast<const float4 *>(src)[i];
+            amax = fmaxf(amax, fmaxf(fmaxf(fabsf(t.x), fabsf(t.y)), fmaxf(fabsf(t.z), fabsf(t.w))));
+        }
+    } else {
+        for (int64_t i = threadIdx.x; i < k; i += 256) amax = fmaxf(amax, fabsf(src[i]));
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
@@ -126,12 +130,12 @@ __global__ void __launch_bounds__(256) gp_x_split_kernel(const float *__restrict
     const float up = __int_as_float((127 + e) << 23);  // e in [-113, 126]
     if (threadIdx.x == 0) scale[row] = __int_as_float((127 - e) << 23);
     for (int64_t o8 = threadIdx.x; o8 < k / 8; o8 += 256) {
-        const float *s = src + (o8 >> 2) * 32;
-        const uint8_t *perm = kGpPerm[order] + (o8 & 3) * 8;
+        float v[8];
+        load_permuted8(src + (o8 >> 2) * 32, (int)(o8 & 3), order, vec, v);
         uint32_t wh[4], wl[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const float a = s[perm[2 * j]] * up, b = s[perm[2 * j + 1]] * up;
+            const float a = v[2 * j] * up, b = v[2 * j + 1] * up;
             const __half2 h = __floats2half2_rn(a, b);
             const __half2 l = __floats2half2_rn(a - __low2float(h), b - __high2float(h));
             wh[j] = *reinterpret_cast<const uint32_t *>(&h);

@@ -562,14 +562,13 @@ cq_status launch_gemm(cq_ctx *ctx, int qtype, int order, int actmode, const floa
     if ((reinterpret_cast<uintptr_t>(w) & 1) != 0 || (reinterpret_cast<uintptr_t>(x) & 3) != 0 || (reinterpret_cast<uintptr_t>(y) & 3) != 0)
         return cq_fail(ctx, CQ_ERR_INVALID_ARG, "gemm: misaligned pointer");
     if (m > 0x7FFFFFFF || n > 0x7FFFFFFF || k > 0x7FFFFFFF) return cq_fail(ctx, CQ_ERR_TOO_LARGE, "gemm: dimension beyond 2^31");
-    // CTA pairs that dequantize raw blocks into tensor memory (gemm_pair_tmem.cu), n 11008 x k 4096, this kernel against what
-    // served the batch before, us: 32 rows 17.7 / 19.1 (Q4_0), 128 rows 23.8 / 28.6, 200 rows 34 / 56, 512 rows 57 / 88, 1024 rows
-    // 100 / 113 (Q8_0: 105 / 125).  Two lines: past 1024 rows the f16 copy of W, made once, costs less than dequantizing W
-    // again for every 128 rows (2048 rows: 187 / 170); up to 64 rows of a large matrix the narrow kernel's loads are the
-    // quicker ones (64 rows x 20480 x 8192: 44.5 / 43.0, Q8_0 58.5 / 47.0; 22016 x 4096: 28.7 / 29.9, Q8_0 37.7 / 32.6), so
-    // there the pairs take shares of up to 9 (Q8_0: 5) of its work items per SM.
+    // CTA pairs that dequantize raw blocks into tensor memory (gemm_pair_tmem.cu), n 11008 x k 4096, this kernel against the other
+    // routes, us: 128 rows 23.8 / 28.6, 200 rows 34 / 56, 600 rows 64 / 80 (Q8_0: 74 / 84).  Its lines: past 1024 rows (Q8_0: 768)
+    // the f16 copy of W, made once, costs less than dequantizing W again for every 128 rows (1024 rows 100 / 106, Q8_0 117 / 110;
+    // 1300 rows 136 / 129, Q8_0 159 / 135); up to 32 rows the narrow kernel's loads are the quicker ones (16 rows 17.3 / 15.0), up
+    // to 64 only on larger matrices (64 rows 20.1 / 21.1; 22016 x 4096 27.7 / 27.3, Q8_0 37.5 / 32.2).
     const int64_t items_per_sm = ((n + 255) / 256) * (k / 256) / ctx->sm_count;
-    const bool pairs_win = m <= 1024 && (m > 64 || items_per_sm < (qtype == CQ_Q4_0 ? 10 : 6));
+    const bool pairs_win = m <= (qtype == CQ_Q4_0 ? 1024 : 768) && (m > 64 || (m > 32 && items_per_sm < 6));
     if (ctx->tune.gemm_variant == 0 && !ctx->tune.gemm_cache_weights && gemm_pair_tmem_supported(qtype, k, w) &&
         (ctx->tune.gemm_fused_dequant == 2 || (ctx->tune.gemm_fused_dequant == 1 && pairs_win)))
         return launch_gemm_pair_tmem(ctx, qtype, order, false, x, m, k, ldx, w, n, y, ldy);

@@ -114,7 +114,7 @@ cq_status cq_ctx_set_option(cq_ctx *ctx, const char *key, int64_t value);
  * GEMM has seen: the weights must then stay unchanged, or be rewritten only through cq_* entry points, or
  * cq_invalidate_weight_cache must be called); gemm_pair (1, default: CQ_ACT_F16 batches that work from an f16 copy
  * of W run 256 x 256 tiles on CTA pairs; 0: 128 x 256 tiles per CTA); gemm_fused_dequant (1, default: Q4_0 and Q8_0
- * batches of up to 1024 rows in CQ_ACT_F16 dequantize the raw blocks inside a CTA-pair GEMM where that is quicker than
+ * batches of 33 to 1024 rows in CQ_ACT_F16 dequantize the raw blocks inside a CTA-pair GEMM where that is quicker than
  * the other routes; 2: at every batch size; 0: never); gemm_int8 (1, default: batches of i8_min_rows_q8_1 (3) or more
  * rows in CQ_ACT_Q8_1 and of i8_min_rows_f32 (3) or more in CQ_ACT_F32 run on the tensor cores, one
  * weight pass per batch; 0: the decode kernels, up to eight rows a pass); split_min_rows (9, default: CQ_ACT_F32

@@ -287,8 +287,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
         }
     } else if (warp == 1) {
         // ---- first MMA issuer: S(t) = Q K(t)^T, as far ahead as the K ring and the score slot allow ----------------------
-        // (one thread issues an M 128 x N 128 x K 16 instruction every ~100 cycles, the tensor pipe needs 64: with the two
-        // products on one thread the issue was the tile's longest role, with a thread each they run side by side)
+        // (with the two products on one issuing warp the issue was the tile's longest role, with a warp each they run side by side)
         {  // the whole warp runs the loop, one lane issues
             constexpr uint32_t idesc_s = idesc_16(FA_M, FA_N, BF16);
             const uint32_t q_addr = smem_u32(sm_q);

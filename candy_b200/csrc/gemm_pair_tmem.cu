@@ -20,9 +20,10 @@
 //              slab into its shared memory (B operand): the slab crosses L2 once per pair
 //   warp 0     TMA, X slabs of 128 k (completion counted on the leader's barrier)
 //   warp 1     TMA, raw blocks: [128 rows x 144 / 272 B] per 256 k
-//   warps 2,3  of the leader: one MMA-issuing lane each (one thread starts an M 256 x N 128 MMA only every ~100 cycles, the
-//              pipe wants one every 64).  SPLIT: one issues Xhi Whi, the other the two corrections; else they take
-//              alternate K = 16 steps.  Each has its own accumulator.
+//   warps 2,3  of the leader: MMA issue.  The whole warp runs the loop and one lane issues: a loop that a lane runs alone starts
+//              an MMA only every ~100-150 cycles, the pipe wants one every 64 (512 rows x 11008 x 4096, SPLIT: 125 -> 109 us).
+//              SPLIT: one warp issues Xhi Whi, the other the two corrections; else they take alternate K = 16 steps.  Each
+//              has its own accumulator.
 //   DQ warps   groups of four (128 rows); group g owns A buffer g and converts every G-th stage of 128 k, so a group
 //              converts while the tensor core works on the other buffers
 //   8 warps    epilogue: lane = weight row, so a batch row's outputs leave in 128-byte runs

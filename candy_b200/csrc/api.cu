@@ -208,6 +208,7 @@ cq_status cq_ctx_set_option(cq_ctx *ctx, const char *key, int64_t value) {
     else if (!strcmp(key, "comm_cluster")) t.comm_cluster = (int)value;
     else if (!strcmp(key, "gemm_int8")) t.gemm_int8 = (int)value;
     else if (!strcmp(key, "split_min_rows")) t.split_min_rows = (int)value;
+    else if (!strcmp(key, "split_min_rows_q8_1")) t.split_min_rows_q8_1 = (int)value;
     else if (!strcmp(key, "i8_min_rows_f32")) t.i8_min_rows_f32 = (int)value;
     else if (!strcmp(key, "i8_min_rows_q8_1")) t.i8_min_rows_q8_1 = (int)value;
     else if (!strcmp(key, "gemv_mma")) t.gemv_mma = (int)value;
@@ -442,12 +443,20 @@ cq_status cq_qmatmul(cq_ctx *ctx, int qtype, int order, int actmode, const float
     // kernel's planes in brackets: 9 rows 21 (28), 128 rows 37 (104), 512 rows 92 (409); up to eight rows the streaming kernel
     // takes 12.7, or for Q8_0 the planes 18.9 against 21).  Only where the planes served before: an x without 16-byte
     // alignment keeps its plain f32 arithmetic.
-    if (actmode == CQ_ACT_F32 && ctx->tune.split_min_rows > 0 && m >= ctx->tune.split_min_rows && ctx->tune.gemm_int8 && !ctx->fuse.on && ctx->push.world == 0 &&
-        ctx->tune.gemv_variant == 0 && !ctx->tune.force_simple && gemm_pair_tmem_supported(qtype, k, w_blocks_dev) &&
-        qgemm_i8_supported(qtype, k, w_blocks_dev, x_dev, ldx) && m <= (1 << 22)) {
+    const bool on_f16_sums = ctx->tune.gemm_int8 && !ctx->fuse.on && ctx->push.world == 0 && ctx->tune.gemv_variant == 0 && !ctx->tune.force_simple &&
+                             gemm_pair_tmem_supported(qtype, k, w_blocks_dev) && qgemm_i8_supported(qtype, k, w_blocks_dev, x_dev, ldx) && m <= (1 << 22);
+    if (actmode == CQ_ACT_F32 && ctx->tune.split_min_rows > 0 && m >= ctx->tune.split_min_rows && on_f16_sums) {
         s = launch_gemm_pair_tmem(ctx, qtype, order, true, x_dev, m, k, ldx, w_blocks_dev, n, y_dev, ldy);
         // captured without the scratch for its operands (4 m k bytes), or no memory for it: the planes below do with about half
         if (!(s == CQ_ERR_INVALID_ARG && cq_stream_capturing(ctx)) && s != CQ_ERR_NOMEM) return s;
+    }
+    // CQ_ACT_Q8_1 from 33 rows on: the same with one product per weight block, scaled in f32 (us, integer dots below in brackets:
+    // n 11008 x k 4096, Q4_0 / Q8_0, 33 rows 32 (44) / 29 (36), 100 rows 39 (73) / 39 (64), 300 rows 85 (217) / 81 (188); 700 x
+    // 1024, 33 rows 12.2 (13.2) / 11.2 (11.5).  32 rows are even there, 30 (31) / 26.5 (27.6), but 4096 x 14336 43 (39) / 38 (33).)
+    if (actmode == CQ_ACT_Q8_1 && ctx->tune.split_min_rows_q8_1 > 0 && m >= ctx->tune.split_min_rows_q8_1 && on_f16_sums) {
+        s = launch_gemm_blocks(ctx, qtype, order, x_dev, m, k, ldx, w_blocks_dev, n, y_dev, ldy);
+        // (captured without the scratch for its operands, no memory for them, or too many tiles in one launch: the integer dots)
+        if (!(s == CQ_ERR_INVALID_ARG && cq_stream_capturing(ctx)) && s != CQ_ERR_NOMEM && s != CQ_ERR_TOO_LARGE) return s;
     }
     // Integer dots on the tensor cores: one weight pass for the whole batch, in the activation mode's own numerics.
     if (actmode != CQ_ACT_F16 && ctx->tune.gemm_int8 && !ctx->fuse.on && ctx->push.world == 0 && ctx->tune.gemv_variant == 0 &&

@@ -49,6 +49,7 @@ struct GemvTuning {
     int gemm_pair = 1;           // m > 128: 256 x 256 tiles on CTA pairs (cta_group::2) instead of 128 x 256 per CTA
     int gemm_fused_dequant = 1;  // CQ_ACT_F16, Q4_0 / Q8_0: the CTA-pair kernel that dequantizes in place (1: where it is the quicker one, 2: every batch of nine and more, 0: never)
     int split_min_rows = 9;      // CQ_ACT_F32 batches of this many rows: both operands as sums of two f16 numbers (0: never)
+    int split_min_rows_q8_1 = 33; // CQ_ACT_Q8_1 batches of this many rows: products of f16 numbers per block instead of integer dots (0: never)
     int i8_min_rows_f32 = 3;
     int i8_min_rows_q8_1 = 3;
     int gemv_mma = 3;       // CQ_ACT_F32, Q4_0: batches of this many rows up to 8 take the single-launch mma.sync kernel (0: never)
@@ -193,6 +194,9 @@ cq_status launch_gemv_f32(cq_ctx *ctx, int qtype, int order, const float *x, int
 bool gemm_pair_tmem_supported(int qtype, int64_t k, const void *w);
 cq_status launch_gemm_pair_tmem(cq_ctx *ctx, int qtype, int order, bool split, const float *x, int64_t m, int64_t k, int64_t ldx, const void *w, int64_t n,
                                 float *y, int64_t ldy);
+// CQ_ACT_Q8_1 batches, a product per weight block and its scale in f32 (gemm_blocks.cu).  Supported where the two kernels above and below are.
+cq_status launch_gemm_blocks(cq_ctx *ctx, int qtype, int order, const float *x, int64_t m, int64_t k, int64_t ldx, const void *w, int64_t n, float *y,
+                             int64_t ldy);
 cq_status launch_gemm(cq_ctx *ctx, int qtype, int order, int actmode, const float *x, int64_t m, int64_t k,
                       int64_t ldx, const void *w, int64_t n, float *y, int64_t ldy);
 

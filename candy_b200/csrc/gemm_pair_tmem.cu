@@ -39,14 +39,11 @@
 //
 // SPLIT and huge scales: f16 holds 65504.  A thread that meets a scale whose products could pass that (or inf / NaN) marks
 // its weight row for the piece of work at hand, and the epilogue computes marked rows of it from the blocks in plain f32.
-#include "common.cuh"
-#include "tcgen05.cuh"
+#include "gemm_raw.cuh"
 
 namespace {
 
-constexpr int GP_ROWS = 128;    // weight rows per CTA
 constexpr int GP_TILE = 256;    // weight rows per pair
-constexpr int GP_CHUNK = 256;   // values of k per work item and raw stage; an A / X stage is half of it
 constexpr int GP_EPW = 8;       // epilogue warps
 constexpr int GP_LEG = 16;      // SPLIT: chunks that the tensor core adds up before an f32 addition does (see above)
 
@@ -68,20 +65,6 @@ struct GpCfg {
     static constexpr size_t kSmem = (size_t)kWStages * kWBytes + (size_t)kXStages * kXBytes + 1024 + 8 * kBars + 16 + 4 * GP_ROWS;
     static constexpr int kACol0 = 256;                         // accumulators: two of NB columns at 0
     static_assert(kSmem <= 232448 && 2 * NB <= kACol0 && kACol0 + kGroups * kACols <= 512, "shared / tensor memory");
-};
-
-struct GpParams {
-    float *y;
-    int64_t ldy;
-    float *part;           // [2 * pairs][NB][256]
-    const float *xscale;   // SPLIT: 2^-e of each batch row, negative for rows to be computed in plain f32
-    const float *x;        // SPLIT: the operands as given, for rows computed in plain f32
-    const uint8_t *w;
-    const float *bias;     // [n] or null
-    int64_t ldx;
-    int m, n, k, order;
-    int mtiles, nchunks, total, per_pair;
-    int *err;
 };
 
 // ---- activation pre-passes ---------------------------------------------------------------------------------
@@ -166,40 +149,6 @@ __global__ void __launch_bounds__(256) gp_x_split_kernel(const float *__restrict
     if (threadIdx.x == 0) scale[row] = (low ? -1.0f : 1.0f) * __int_as_float((127 - e) << 23);
 }
 
-// y of the tiles whose k range several pairs shared: their partial tiles, added in pair order.  Block = (tile, four batch rows).
-template <int NB>
-__global__ void __launch_bounds__(256) gp_sum_kernel(const GpParams p) {
-    pdl_launch_dependents();
-    pdl_wait_prior();
-    const int t = blockIdx.x, lc = blockIdx.y * 4 + (threadIdx.x >> 6);
-    const int group = t / p.mtiles, col = (t - group * p.mtiles) * NB + lc;
-    const int first = (t * p.nchunks) / p.per_pair, last = ((t + 1) * p.nchunks - 1) / p.per_pair;
-    if (first == last || col >= p.m) return;  // one pair had the whole k range and wrote y itself
-    const int r = (threadIdx.x & 63) * 4;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int c = first; c <= last; ++c) {
-        const int slot = 2 * c + (((c * p.per_pair) / p.nchunks == t) ? 0 : 1);
-        const float4 v = *reinterpret_cast<const float4 *>(p.part + ((int64_t)slot * NB + lc) * GP_TILE + r);
-        acc.x += v.x, acc.y += v.y, acc.z += v.z, acc.w += v.w;
-    }
-    const int64_t j = (int64_t)group * GP_TILE + r;
-    if (p.bias) {
-        if (j < p.n) acc.x += p.bias[j];
-        if (j + 1 < p.n) acc.y += p.bias[j + 1];
-        if (j + 2 < p.n) acc.z += p.bias[j + 2];
-        if (j + 3 < p.n) acc.w += p.bias[j + 3];
-    }
-    float *dst = p.y + (int64_t)col * p.ldy + j;
-    if (j + 3 < p.n && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-        *reinterpret_cast<float4 *>(dst) = acc;
-    } else {
-        if (j < p.n) dst[0] = acc.x;
-        if (j + 1 < p.n) dst[1] = acc.y;
-        if (j + 2 < p.n) dst[2] = acc.z;
-        if (j + 3 < p.n) dst[3] = acc.w;
-    }
-}
-
 // q (an f16 pair of whole numbers) times the scale: the rounded product, and what the rounding took off (exact)
 template <bool SPLIT>
 __device__ __forceinline__ void gp_scale(__half2 q, __half2 d2, uint32_t &hi, uint32_t &lo) {
@@ -210,28 +159,19 @@ __device__ __forceinline__ void gp_scale(__half2 q, __half2 d2, uint32_t &hi, ui
         lo = *reinterpret_cast<const uint32_t *>(&l);
     }
 }
-// Eight nibbles -> four pairs (v0,v4)(v1,v5)(v2,v6)(v3,v7): 1024 + q assembled by one mask-or, 1032 taken off exactly.
 template <bool SPLIT>
 __device__ __forceinline__ void gp_dequant_q4(uint32_t n, __half2 d2, uint32_t *hi, uint32_t *lo) {
-    const __half2 k1032 = __halves2half2(__ushort_as_half(0x6408), __ushort_as_half(0x6408));
-    const __half2 k16th = __halves2half2(__ushort_as_half(0x2C00), __ushort_as_half(0x2C00));
-    const __half2 km72 = __halves2half2(__ushort_as_half(0xD480), __ushort_as_half(0xD480));
-    const uint32_t n8 = n >> 8;
-    uint32_t t0 = (n & 0x000F000Fu) | 0x64006400u, t1 = (n & 0x00F000F0u) | 0x64006400u;
-    uint32_t t2 = (n8 & 0x000F000Fu) | 0x64006400u, t3 = (n8 & 0x00F000F0u) | 0x64006400u;
-    gp_scale<SPLIT>(__hsub2(*reinterpret_cast<__half2 *>(&t0), k1032), d2, hi[0], lo[0]);
-    gp_scale<SPLIT>(__hfma2(*reinterpret_cast<__half2 *>(&t1), k16th, km72), d2, hi[1], lo[1]);
-    gp_scale<SPLIT>(__hsub2(*reinterpret_cast<__half2 *>(&t2), k1032), d2, hi[2], lo[2]);
-    gp_scale<SPLIT>(__hfma2(*reinterpret_cast<__half2 *>(&t3), k16th, km72), d2, hi[3], lo[3]);
+    __half2 q[4];
+    gp_numbers_q4(n, q);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) gp_scale<SPLIT>(q[j], d2, hi[j], lo[j]);
 }
-// Four int8 -> two pairs, natural order.
 template <bool SPLIT>
 __device__ __forceinline__ void gp_dequant_q8(uint32_t n, __half2 d2, uint32_t *hi, uint32_t *lo) {
-    const __half2 k1152 = __halves2half2(__ushort_as_half(0x6480), __ushort_as_half(0x6480));
-    const uint32_t u = n ^ 0x80808080u;
-    uint32_t t0 = __byte_perm(u, 0x64646464u, 0x4140), t1 = __byte_perm(u, 0x64646464u, 0x4342);
-    gp_scale<SPLIT>(__hsub2(*reinterpret_cast<__half2 *>(&t0), k1152), d2, hi[0], lo[0]);
-    gp_scale<SPLIT>(__hsub2(*reinterpret_cast<__half2 *>(&t1), k1152), d2, hi[1], lo[1]);
+    __half2 q[2];
+    gp_numbers_q8(n, q);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) gp_scale<SPLIT>(q[j], d2, hi[j], lo[j]);
 }
 
 __device__ __forceinline__ void tc_mma_f16_ts_pair(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
@@ -295,7 +235,7 @@ __global__ void __launch_bounds__(GpCfg<QT, SPLIT, NB>::kThreads, 1)
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
     const int pair = blockIdx.x >> 1;
-    const int g0 = pair * p.per_pair, g1 = min(g0 + p.per_pair, p.total);
+    const int g0 = pair * p.per_share, g1 = min(g0 + p.per_share, p.total);
     const int nst = 2 * (g1 - g0);  // A / X stages of this share
 
     if (threadIdx.x == 0) {
@@ -626,54 +566,6 @@ __global__ void __launch_bounds__(GpCfg<QT, SPLIT, NB>::kThreads, 1)
     if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
 }
 
-// Raw blocks as a 2-D tensor of 2-byte elements, box = 256 values of k x 128 rows.
-bool gp_w_map(CUtensorMap *map, const void *w, int64_t n, int64_t row_bytes, int row_chunk) {
-    EncodeTiledFn fn = encode_tiled_fn();
-    if (!fn) return false;
-    cuuint64_t dims[2] = {(cuuint64_t)(row_bytes / 2), (cuuint64_t)n};
-    cuuint64_t strides[1] = {(cuuint64_t)row_bytes};
-    cuuint32_t box[2] = {(cuuint32_t)(row_chunk / 2), (cuuint32_t)GP_ROWS};
-    cuuint32_t estr[2] = {1, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void *>(w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-// Activations as [hi / lo][k / 64][m][64]: ONE copy then brings a whole stage (128 k of `rows` batch rows, both halves of a
-// split) as the 64-wide swizzled boxes the MMA reads; one thread starts a copy only every few hundred cycles.
-bool gp_x_map(CUtensorMap *map, const void *x16, int64_t m, int64_t k, size_t lo_offset, int rows) {
-    EncodeTiledFn fn = encode_tiled_fn();
-    if (!fn) return false;
-    const int parts = lo_offset ? 2 : 1;
-    cuuint64_t dims[4] = {64u, (cuuint64_t)m, (cuuint64_t)(k / 64), (cuuint64_t)parts};
-    cuuint64_t strides[3] = {(cuuint64_t)k * 2, 128u, lo_offset ? (cuuint64_t)lo_offset : (cuuint64_t)k * 2};
-    cuuint32_t box[4] = {64u, (cuuint32_t)rows, 2u, (cuuint32_t)parts};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void *>(x16), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-template <typename Kern, typename... Args>
-cq_status gp_launch(cq_ctx *ctx, Kern kern, dim3 grid, int block, size_t smem, bool cluster, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = ctx->stream;
-    cudaLaunchAttribute attr[2];
-    int na = 0;
-    if (ctx->tune.pdl) {
-        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[na++].val.programmaticStreamSerializationAllowed = 1;
-    }
-    if (cluster) {
-        attr[na].id = cudaLaunchAttributeClusterDimension;
-        attr[na].val.clusterDim.x = 2, attr[na].val.clusterDim.y = 1, attr[na++].val.clusterDim.z = 1;
-    }
-    cfg.attrs = attr;
-    cfg.numAttrs = na;
-    CQ_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, args...));
-    return CQ_OK;
-}
-
 template <int QT, bool SPLIT, int NB>
 cq_status gp_run(cq_ctx *ctx, const float *x, int64_t m, int64_t k, int64_t ldx, int order, const void *w, int64_t n, float *y, int64_t ldy) {
     using Cfg = GpCfg<QT, SPLIT, NB>;
@@ -696,22 +588,12 @@ cq_status gp_run(cq_ctx *ctx, const float *x, int64_t m, int64_t k, int64_t ldx,
     GpParams p = {};
     p.y = y, p.ldy = ldy, p.x = x, p.w = static_cast<const uint8_t *>(w), p.ldx = ldx;
     p.m = (int)m, p.n = (int)n, p.k = (int)k, p.order = order, p.err = ctx->dev_err_devptr, p.bias = ctx->bias;
-    p.mtiles = (int)((m + NB - 1) / NB);
-    p.nchunks = (int)(k / GP_CHUNK);
-    const int64_t tiles = ((n + GP_TILE - 1) / GP_TILE) * (int64_t)p.mtiles, total = tiles * p.nchunks;
-    if (total > 0x3FFFFFFF / 2) return cq_fail(ctx, CQ_ERR_TOO_LARGE, "gemm: too many tiles");
-    int64_t per = (total + max_pairs - 1) / max_pairs;
-    if (per < 2) per = total < 2 ? total : 2;
     const size_t x_bytes = (((size_t)m * k * 2) + 1023) & ~size_t(1023);
     const size_t scale_bytes = SPLIT ? (((size_t)m * 4) + 1023) & ~size_t(1023) : 0;
     const size_t operand_bytes = (SPLIT ? 2 : 1) * x_bytes + scale_bytes;
-    auto part_bytes = [&] { return per % p.nchunks != 0 ? (size_t)2 * ((total + per - 1) / per) * NB * GP_TILE * 4 : size_t(0); };
-    // captured with room for the operands but not for partial tiles: whole tiles per pair, which need none
-    if (operand_bytes + part_bytes() > ctx->scratch_bytes && cq_stream_capturing(ctx)) per = (tiles + max_pairs - 1) / max_pairs * p.nchunks;
-    const unsigned pairs = (unsigned)((total + per - 1) / per);
-    p.total = (int)total, p.per_pair = (int)per;
-    const bool shared = per % p.nchunks != 0;
-    cq_status s = cq_reserve_scratch(ctx, operand_bytes + part_bytes());
+    GpShares sh;
+    cq_status s = gp_share_out(ctx, p, GP_TILE, NB, max_pairs, operand_bytes, sh);
+    if (s == CQ_OK) s = cq_reserve_scratch(ctx, operand_bytes + sh.part_bytes);
     if (s != CQ_OK) return s;
     uint8_t *base = static_cast<uint8_t *>(ctx->scratch);
     __half *xh = reinterpret_cast<__half *>(base), *xl = reinterpret_cast<__half *>(base + (SPLIT ? x_bytes : 0));
@@ -719,7 +601,7 @@ cq_status gp_run(cq_ctx *ctx, const float *x, int64_t m, int64_t k, int64_t ldx,
     p.part = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(scale) + scale_bytes);
     p.xscale = scale;
     CUtensorMap tmW, tmX;
-    if (!gp_w_map(&tmW, w, n, (k / kQK) * Cfg::kBlockBytes, Cfg::kRowChunk) || !gp_x_map(&tmX, xh, m, k, SPLIT ? x_bytes : 0, NB / 2))
+    if (!gp_w_map(&tmW, w, n, (k / kQK) * Cfg::kBlockBytes, Cfg::kRowChunk) || !gp_x_map(&tmX, xh, m, k, SPLIT ? x_bytes : 0, NB / 2, 2))
         return cq_fail(ctx, CQ_ERR_CUDA, "gemm: cuTensorMapEncodeTiled failed or is unavailable");
     const int ord = QT == CQ_Q4_0 ? order : 2;
     if (SPLIT) {
@@ -729,8 +611,8 @@ cq_status gp_run(cq_ctx *ctx, const float *x, int64_t m, int64_t k, int64_t ldx,
         s = gp_launch(ctx, gp_x_f16_kernel, dim3((unsigned)((items + 255) / 256 < cap ? (items + 255) / 256 : cap)), 256, 0, false, x, m, k, ldx, ord, xh);
     }
     if (s != CQ_OK) return s;
-    s = gp_launch(ctx, kern, dim3(2 * pairs), Cfg::kThreads, Cfg::kSmem, true, tmW, tmX, p);
-    if (s == CQ_OK && shared) s = gp_launch(ctx, gp_sum_kernel<NB>, dim3((unsigned)tiles, NB / 4), 256, 0, false, p);
+    s = gp_launch(ctx, kern, dim3(2 * sh.shares), Cfg::kThreads, Cfg::kSmem, true, tmW, tmX, p);
+    if (s == CQ_OK && sh.cut) s = gp_launch(ctx, gp_sum_kernel<GP_TILE, NB>, dim3((unsigned)sh.tiles, NB / 4), 256, 0, false, p);
     if (s == CQ_OK && p.bias) ctx->bias_done = true;
     return s;
 }

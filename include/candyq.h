@@ -119,7 +119,8 @@ cq_status cq_ctx_set_option(cq_ctx *ctx, const char *key, int64_t value);
  * rows in CQ_ACT_Q8_1 and of i8_min_rows_f32 (3) or more in CQ_ACT_F32 run on the tensor cores, one
  * weight pass per batch; 0: the decode kernels, up to eight rows a pass); split_min_rows (9, default: CQ_ACT_F32
  * batches of this many rows multiply sums of two f16 numbers, in effect 22-bit operands; 0: the int8 kernel serves
- * them too); attn_variant (decode attention: 1 = one CTA per 32-key chunk for grouped heads instead of split contexts, 2 = never the
+ * them too); split_min_rows_q8_1 (33, default: CQ_ACT_Q8_1 batches of this many rows multiply d8 q8 as sums of two f16
+ * numbers by the weights' whole numbers; 0: always integer dots); attn_variant (decode attention: 1 = one CTA per 32-key chunk for grouped heads instead of split contexts, 2 = never the
  * single-launch cluster kernel of short contexts); comm_poll_limit (polls before the reducing
  * norm gives up on a peer's data, default about one second's worth); comm_cluster; host_zero_copy (see
  * cq_qmatmul_host); fa_transpose_v (1: cq_flash_attention always transposes V into scratch first; 0, default: V tiles
@@ -131,7 +132,7 @@ cq_status cq_ctx_set_option(cq_ctx *ctx, const char *key, int64_t value);
  * protect (reserve up front).
  * What a cq_qmatmul / cq_qlinear call takes of it, in bytes, with m rounded up to a multiple of 128: CQ_ACT_F32 at most
  * 4 m k + 20 MiB (captured with less, 2.25 m k + 10 MiB will do, in the 15-bit block fixed point of smaller batches);
- * CQ_ACT_Q8_1 1.25 m k + 20 MiB; CQ_ACT_F16 2 m k + 40 MiB up to 128 rows of Q4_0 / Q8_0, 2 m k + 20 MiB (captured: 2 m k)
+ * CQ_ACT_Q8_1 4.5 m k + 20 MiB (captured with less, 1.25 m k + 20 MiB will do, in the integer dots of smaller batches); CQ_ACT_F16 2 m k + 40 MiB up to 128 rows of Q4_0 / Q8_0, 2 m k + 20 MiB (captured: 2 m k)
  * up to 768, beyond that and for the other formats 2 k (m + n).
  * Rows that are not multiples of 256 values: where it pays, CQ_ACT_Q8_1 and CQ_ACT_F16 calls multiply copies of W and x with
  * padded rows.  The copies lie in a block of their own (at most 1 GiB; larger matrices take a slower route), which cq_reserve
@@ -194,7 +195,7 @@ cq_status cq_quantize_q8_1(cq_ctx *ctx, const float *x_dev, int64_t m, int64_t k
  * block as 15-bit block fixed point, about 2e-5 of max|y| from the CPU path; larger ones multiply sums of two f16
  * numbers: 22 bits of most activations, at least 15 of the largest value of each 32-block, and sums within 3e-5 of an
  * output's sum |x| |w| at any k, about 4e-6 of max|y| for centred operands; CQ_ACT_Q8_1 batches quantize exactly as quantize_q8_1 does; up to eight rows against Q4_0 run
- * in a single-launch streaming kernel, larger Q8_1 batches in the int8 GEMM);
+ * in a single-launch streaming kernel, batches of up to 32 in the int8 GEMM, larger ones multiply d8 q8 in f16 pieces);
  * CQ_ACT_F16 runs the f16 tensor-core GEMMs (up to eight rows against Q4_0: the single-launch streaming kernel with
  * f16 operands, same rounding of the operands).
  * Preconditions: k % 32 == 0, k >= 32, m, n >= 1, ldx >= k, ldy >= n. */

@@ -41,57 +41,13 @@
 // the tensor maps cannot address (rows not 16-byte aligned) is transposed into context scratch by a small kernel first
 // and read as a K-major V^T (the first form of this kernel did that always: 79.6 us against 58.5 at 32 heads x 2048).
 // Every wait is bounded; tensor memory is always freed.
-#include <cuda_bf16.h>
+#include <algorithm>
 
-#include <cmath>
-
-#include "common.cuh"
-#include "tcgen05.cuh"
+#include "attention.cuh"
 
 namespace {
 
-constexpr int FA_M = 128;   // query rows per CTA
-constexpr int FA_N = 128;   // keys per tile
 constexpr int FA_THREADS = 352;  // TMA warp, first MMA issuer, eight compute warps, second MMA issuer
-
-struct FaParams {
-    void *o;
-    float *lse;             // [b][h][seqlen_q] or null
-    int64_t o_batch_stride, o_row_stride, o_head_stride;
-    int b, h, h_k, seqlen_q, seqlen_k;
-    int causal;
-    float scale_log2;       // softmax_scale * log2(e)
-    float scale;            // softmax_scale
-    int *err;
-};
-
-__device__ __forceinline__ void tma_load_3d(uint32_t smem_dst, const CUtensorMap *map, int c0, int c1, int c2, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_dst),
-        "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
-        : "memory");
-}
-// kind::f16 instruction descriptor with the operand type: f16 (0) or bf16 (1); D f32; both operands K-major.
-__host__ __device__ constexpr uint32_t idesc_16(int mm, int nn, bool bf16) {
-    return (1u << 4) | ((bf16 ? 1u : 0u) << 7) | ((bf16 ? 1u : 0u) << 10) | ((uint32_t)(nn >> 3) << 17) | ((uint32_t)(mm >> 4) << 24);
-}
-
-// 2^x by the special-function unit (relative error about 2^-22; -inf gives 0)
-__device__ __forceinline__ float fast_ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-template <bool BF16>
-__device__ __forceinline__ uint32_t pack2(float a, float b) {
-    if (BF16) {
-        const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-        return *reinterpret_cast<const uint32_t *>(&v);
-    }
-    const __half2 v = __floats2half2_rn(a, b);
-    return *reinterpret_cast<const uint32_t *>(&v);
-}
 
 // V [b][key][h_k][d] (strides in elements) -> Vt [b * h_k][d][sk_pad], 16-bit elements moved as they are.
 __global__ void __launch_bounds__(256) fa_transpose_v_kernel(const uint16_t *__restrict__ v, int64_t bs, int64_t rs, int64_t hs, int h_k, int d, int sk,
@@ -475,7 +431,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
                             p1 = c0 + 1 <= kmax ? p1 : 0.0f;
                         }
                         l2[(i & 1) * 2] += p0, l2[(i & 1) * 2 + 1] += p1;
-                        pk[i] = pack2<BF16>(p0, p1);
+                        pk[i] = pack16<BF16>(p0, p1);
                     }
                     tmem_st16(lane_addr + Cfg::kColP + (uint32_t)(buf * (FA_N / 2) + half * (HC / 2) + c * 16), pk);
                 }
@@ -510,10 +466,10 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
 #pragma unroll
                 for (int c = 0; c < HD / 8; ++c) {
                     uint4 wv;
-                    wv.x = pack2<BF16>(acc[8 * c] * inv, acc[8 * c + 1] * inv);
-                    wv.y = pack2<BF16>(acc[8 * c + 2] * inv, acc[8 * c + 3] * inv);
-                    wv.z = pack2<BF16>(acc[8 * c + 4] * inv, acc[8 * c + 5] * inv);
-                    wv.w = pack2<BF16>(acc[8 * c + 6] * inv, acc[8 * c + 7] * inv);
+                    wv.x = pack16<BF16>(acc[8 * c] * inv, acc[8 * c + 1] * inv);
+                    wv.y = pack16<BF16>(acc[8 * c + 2] * inv, acc[8 * c + 3] * inv);
+                    wv.z = pack16<BF16>(acc[8 * c + 4] * inv, acc[8 * c + 5] * inv);
+                    wv.w = pack16<BF16>(acc[8 * c + 6] * inv, acc[8 * c + 7] * inv);
                     reinterpret_cast<uint4 *>(dst)[c] = wv;
                 }
             }
@@ -524,17 +480,6 @@ __global__ void __launch_bounds__(FA_THREADS, 1)
     if (warp == 1) tmem_dealloc(tmem_base, 512);
 }
 
-// Q / K: [b][row][head][d] with strides in elements -> 4-D map (d, head, row, batch); box = 64 x 1 x 128 x 1.
-bool make_qk_map(CUtensorMap *map, const void *base, bool bf16, int d, int heads, int rows, int batches, int64_t hs, int64_t rs, int64_t bs) {
-    EncodeTiledFn fn = encode_tiled_fn();
-    if (!fn) return false;
-    cuuint64_t dims[4] = {(cuuint64_t)d, (cuuint64_t)heads, (cuuint64_t)rows, (cuuint64_t)batches};
-    cuuint64_t strides[3] = {(cuuint64_t)hs * 2, (cuuint64_t)rs * 2, (cuuint64_t)bs * 2};
-    cuuint32_t box[4] = {64u, 1u, 128u, 1u};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
-    return fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void *>(base), dims, strides, box, estr,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
 // V^T: [b * h_k][d][sk_pad] -> 3-D map (key, d, b * h_k) whose key extent is seqlen_k (keys beyond read as zero); box = 64 keys x d x 1.
 bool make_vt_map(CUtensorMap *map, const void *base, bool bf16, int d, int sk, int sk_pad, int planes) {
     EncodeTiledFn fn = encode_tiled_fn();
@@ -566,6 +511,28 @@ cq_status run_fa(cq_ctx *ctx, const CUtensorMap &tq, const CUtensorMap &tk, cons
     cfg.numAttrs = ctx->tune.pdl ? 1 : 0;
     CQ_CUDA(ctx, cudaLaunchKernelEx(&cfg, fmha_fwd_kernel<D, BF16, VT>, tq, tk, tv, p));
     return CQ_OK;
+}
+
+// Whether two query tiles per CTA are quicker: a step of theirs (one key tile, both query tiles) takes 4/3 of what a key tile takes
+// here (4096 keys, one item per SM: 54 and 42 us), but there are half as many items to fill the SMs with.  Counted is the busiest
+// SM's work: items are dealt out heavy first in rounds, so a full round gives each SM about its middle item, the last one its
+// first.  (us, one / two tiles: 32 heads x 1024 x 1024 causal 17.9 / 19.4, 40 heads x 900 23.5 / 19.3, 16 heads x 2048 26.3 / 32.3,
+// 32 heads x 2048 47.5 / 36.3; without a mask 32 heads x 1024 27.1 / 20.7, 8 heads x 2048 25.2 / 32.3.)
+bool two_tiles_win(const FaParams &p, int sms) {
+    const int64_t hb = (int64_t)p.h * p.b;
+    if (p.seqlen_q <= FA_M) return false;
+    auto busiest = [&](int64_t rows) {  // key tiles, with `rows` query rows per item
+        const int64_t nq = (p.seqlen_q + rows - 1) / rows, items = nq * hb, all = (p.seqlen_k + FA_N - 1) / FA_N;
+        int64_t sum = 0;
+        for (int64_t first = 0; first < items; first += sms) {
+            const int64_t at = first + sms <= items ? first + sms / 2 : first, last = std::min<int64_t>((nq - at / hb) * rows, p.seqlen_q);  // rows before this
+            const int64_t lim = p.causal ? last + p.seqlen_k - p.seqlen_q : p.seqlen_k;  // keys that the item's last row sees
+            sum += std::max<int64_t>(0, std::min(all, (lim + FA_N - 1) / FA_N));
+        }
+        return sum;
+    };
+    if ((p.seqlen_q + 2 * FA_M - 1) / (2 * FA_M) * hb >= 16 * (int64_t)sms) return true;  // both fill the SMs
+    return 4 * busiest(2 * FA_M) < 3 * busiest(FA_M);
 }
 
 }  // namespace
@@ -636,6 +603,9 @@ cq_status cq_flash_attention(cq_ctx *ctx, void *q_ptr, void *k_ptr, void *v_ptr,
     // persistent CTAs, one per SM (the kernel's shared memory allows no more), each walking its share of the work items
     const int64_t items = (int64_t)((seqlen_q + FA_M - 1) / FA_M) * h * b;
     const dim3 grid((unsigned)(items < ctx->sm_count ? items : ctx->sm_count));
+    if (v_direct && ctx->tune.fa_two_tiles && softmax_scale > 0.0f && seqlen_k <= (bf ? 65536u : 16384u) &&
+        (ctx->tune.fa_two_tiles == 2 || two_tiles_win(p, ctx->sm_count)))
+        return launch_fmha_two_tiles(ctx, tq, tk, tv, p, (int)d, bf);
     if (v_direct) {
         if (d == 128) return bf ? run_fa<128, true, false>(ctx, tq, tk, tv, p, grid) : run_fa<128, false, false>(ctx, tq, tk, tv, p, grid);
         return bf ? run_fa<64, true, false>(ctx, tq, tk, tv, p, grid) : run_fa<64, false, false>(ctx, tq, tk, tv, p, grid);

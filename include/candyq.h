@@ -123,7 +123,8 @@ cq_status cq_ctx_set_option(cq_ctx *ctx, const char *key, int64_t value);
  * numbers by the weights' whole numbers; 0: always integer dots); attn_variant (decode attention: 1 = one CTA per 32-key chunk for grouped heads instead of split contexts, 2 = never the
  * single-launch cluster kernel of short contexts); comm_poll_limit (polls before the reducing
  * norm gives up on a peer's data, default about one second's worth); comm_cluster; host_zero_copy (see
- * cq_qmatmul_host); fa_transpose_v (1: cq_flash_attention always transposes V into scratch first; 0, default: V tiles
+ * cq_qmatmul_host); fa_two_tiles (1, default: cq_flash_attention works on two tiles of 128 query rows per
+ * CTA where that is quicker; 0: never; 2: wherever it can); fa_transpose_v (1: cq_flash_attention always transposes V into scratch first; 0, default: V tiles
  * are read in place when V is 16-byte aligned with strides that are multiples of 8 elements). */
 /* Grows the context's scratch memory to at least `bytes` now, so that no later call has to (scratch cannot
  * grow while the stream is being captured: such a call fails with CQ_ERR_INVALID_ARG and leaves the capture

@@ -61,6 +61,7 @@ SIGNATURES = {
     "cq_qmatmul": [_vp, _int, _int, _int, _vp, _i64, _i64, _i64, _vp, _i64, _vp, _i64],
     "cq_qlinear": [_vp, _int, _int, _int, _vp, _i64, _i64, _i64, _vp, _i64, _vp, _vp, _i64],
     "cq_qmatmul_host": [_vp, _int, _int, _int, _vp, _i64, _i64, _vp, _i64, _vp],
+    "cq_qlinear_host": [_vp, _int, _int, _int, _vp, _i64, _i64, _vp, _i64, _vp, _vp],
     "cq_qmatmul_q8_1_static": [_vp, _int, _int, _vp, _i64, _i64, _i64, _vp, _i64, _vp, _i64],
     "cq_rand_normal": [_vp, _vp, _i64, C.c_float, C.c_float, C.c_uint64],
     "cq_rand_uniform": [_vp, _vp, _i64, C.c_float, C.c_float, C.c_uint64],

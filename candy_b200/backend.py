@@ -24,6 +24,7 @@ __all__ = ["CudaDevice", "CudaStorage", "QStorage", "QLinear", "Q4_0", "Q4_1", "
 
 
 STAGING_BYTES = 64 << 20  # that a device keeps between host calls
+HOST_CALL_BYTES = 1 << 20  # a host call's input and result up to this size go through cq_qlinear_host
 
 
 class CudaDevice:
@@ -275,6 +276,11 @@ class QLinear:
         w, dev = self.w, self.w.device()
         lib, ctx = dev._lib, dev.ctx
         x, y = np.ascontiguousarray(x), np.empty((rows, w.n), dtype=np.float32)
+        if x.nbytes <= HOST_CALL_BYTES and y.nbytes <= HOST_CALL_BYTES:
+            # the whole call in the library, through its page-locked blocks and with one wait
+            dev._check(lib.cq_qlinear_host(ctx, w.qtype, w.order, self.actmode, x.ctypes.data, rows, w.k, w.buf.ptr, w.n,
+                                           None if self._b_dev is None else self._b_dev.ptr, y.ctypes.data), "linear")
+            return y.reshape(*bs, w.n)
         xs, ys = dev._stage(x.nbytes), (0, None)
         try:
             ys = dev._stage(y.nbytes)

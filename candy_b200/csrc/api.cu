@@ -174,6 +174,8 @@ cq_status cq_ctx_destroy(cq_ctx *ctx) {
     for (auto &kv : ctx->w16_cache) cudaFree(kv.second);
     if (ctx->xfer_x) cudaFree(ctx->xfer_x);
     if (ctx->xfer_y) cudaFree(ctx->xfer_y);
+    if (ctx->pin_x) cudaFreeHost(ctx->pin_x);
+    if (ctx->pin_y) cudaFreeHost(ctx->pin_y);
     if (ctx->ev_start) cudaEventDestroy(ctx->ev_start);
     if (ctx->ev_stop) cudaEventDestroy(ctx->ev_stop);
     if (ctx->dev_err) cudaFreeHost(ctx->dev_err);
@@ -519,6 +521,44 @@ cq_status cq_qlinear_fused(cq_ctx *ctx, int qtype, int order, const float *x_dev
 
 cq_status cq_qmatmul_host(cq_ctx *ctx, int qtype, int order, int actmode, const float *x_host, int64_t m, int64_t k,
                           const void *w_blocks_dev, int64_t n, float *y_host) {
+    return cq_qlinear_host(ctx, qtype, order, actmode, x_host, m, k, w_blocks_dev, n, nullptr, y_host);
+}
+
+// Page-locked blocks of the context for host buffers that are not page-locked themselves.  A copy between pageable memory and
+// the device goes through the driver's own block and waits for it twice: 17 of the 46 us that a 4096 x 4096 Q8_0 linear took on
+// one row.  Copying into such a block first and letting the copy engine, or the kernel's stores, work on that leaves one wait.
+// A megabyte a direction is kept; above that the driver's way costs little beside the transfer.
+static constexpr size_t kPinnedMax = size_t(1) << 20;
+
+static void *pinned_block(cq_ctx *ctx, void **block, size_t *have, size_t bytes) {
+    if (bytes > kPinnedMax) return nullptr;
+    if (bytes > *have) {
+        if (*block) cudaFreeHost(*block);
+        *block = nullptr, *have = 0;
+        size_t want = 64 << 10;
+        while (want < bytes) want *= 2;
+        if (cudaHostAlloc(block, want, cudaHostAllocDefault) != cudaSuccess) {
+            cudaGetLastError();
+            *block = nullptr;
+            return nullptr;
+        }
+        *have = want;
+    }
+    return *block;
+}
+
+static cudaMemoryType memory_type(const void *p, void **device) {
+    cudaPointerAttributes pa;
+    if (cudaPointerGetAttributes(&pa, p) != cudaSuccess) {
+        cudaGetLastError();
+        return cudaMemoryTypeUnregistered;
+    }
+    *device = pa.devicePointer;
+    return pa.type;
+}
+
+cq_status cq_qlinear_host(cq_ctx *ctx, int qtype, int order, int actmode, const float *x_host, int64_t m, int64_t k,
+                          const void *w_blocks_dev, int64_t n, const float *bias_dev, float *y_host) {
     CQ_ENTER(ctx);
     cq_status s = check_matmul_args(ctx, qtype, order, actmode, x_host, m, k, k, w_blocks_dev, n, y_host, n);
     if (s != CQ_OK) return s;
@@ -535,22 +575,34 @@ cq_status cq_qmatmul_host(cq_ctx *ctx, int qtype, int order, int actmode, const 
         CQ_CUDA(ctx, cq_device_malloc(ctx, &ctx->xfer_y, yb));
         ctx->xfer_y_bytes = yb;
     }
-    CQ_CUDA(ctx, cudaMemcpyAsync(ctx->xfer_x, x_host, xb, cudaMemcpyHostToDevice, ctx->stream));
+    const void *x_src = x_host;
+    void *y_block = nullptr, *mapped = nullptr, *y_mapped = nullptr;
+    if (memory_type(x_host, &mapped) == cudaMemoryTypeUnregistered) {
+        if (void *block = pinned_block(ctx, &ctx->pin_x, &ctx->pin_x_bytes, xb)) x_src = memcpy(block, x_host, xb);
+    }
+    CQ_CUDA(ctx, cudaMemcpyAsync(ctx->xfer_x, x_src, xb, cudaMemcpyHostToDevice, ctx->stream));
     // A result buffer in pinned host memory is written by the kernel itself (it is addressable from the device):
     // no copy out, one submission less.  Only for the row-streaming kernels (m <= 8), which store every result
-    // once and coalesced, and only for small results: the stores cross PCIe.
-    float *y_direct = nullptr;
-    if (m <= 8 && ctx->tune.host_zero_copy > 0 && yb <= (size_t)ctx->tune.host_zero_copy) {
-        cudaPointerAttributes pa;
-        if (cudaPointerGetAttributes(&pa, y_host) == cudaSuccess && pa.type == cudaMemoryTypeHost && pa.devicePointer)
-            y_direct = static_cast<float *>(pa.devicePointer);
-        else
-            cudaGetLastError();
+    // once and coalesced, and only for small results: the stores cross PCIe.  (A bias may be added by a kernel of its own.)
+    switch (memory_type(y_host, &mapped)) {
+        case cudaMemoryTypeHost: y_mapped = mapped; break;
+        case cudaMemoryTypeUnregistered:
+            y_block = pinned_block(ctx, &ctx->pin_y, &ctx->pin_y_bytes, yb);
+            if (y_block && memory_type(y_block, &mapped) == cudaMemoryTypeHost) y_mapped = mapped;
+            break;
+        default: break;
     }
-    s = cq_qmatmul(ctx, qtype, order, actmode, (const float *)ctx->xfer_x, m, k, k, w_blocks_dev, n, y_direct ? y_direct : (float *)ctx->xfer_y, n);
-    if (s != CQ_OK) return s;
-    if (!y_direct) CQ_CUDA(ctx, cudaMemcpyAsync(y_host, ctx->xfer_y, yb, cudaMemcpyDeviceToHost, ctx->stream));
-    return cq_synchronize(ctx);
+    const bool in_place = y_mapped && m <= 8 && !bias_dev && ctx->tune.host_zero_copy > 0 && yb <= (size_t)ctx->tune.host_zero_copy;
+    s = cq_qlinear(ctx, qtype, order, actmode, (const float *)ctx->xfer_x, m, k, k, w_blocks_dev, n, bias_dev,
+                   in_place ? static_cast<float *>(y_mapped) : (float *)ctx->xfer_y, n);
+    if (s != CQ_OK) {
+        cudaStreamSynchronize(ctx->stream);  // the copy in may still read the block, or the caller's buffer
+        return s;
+    }
+    if (!in_place) CQ_CUDA(ctx, cudaMemcpyAsync(y_block ? y_block : y_host, ctx->xfer_y, yb, cudaMemcpyDeviceToHost, ctx->stream));
+    s = cq_synchronize(ctx);
+    if (s == CQ_OK && y_block) memcpy(y_host, y_block, yb);
+    return s;
 }
 
 struct cq_graph {

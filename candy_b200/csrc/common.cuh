@@ -101,6 +101,9 @@ struct cq_ctx {
     void *xfer_x = nullptr;       // device staging used by cq_qmatmul_host
     void *xfer_y = nullptr;
     size_t xfer_x_bytes = 0, xfer_y_bytes = 0;
+    void *pin_x = nullptr;        // page-locked staging of cq_qlinear_host, a megabyte each at most
+    void *pin_y = nullptr;
+    size_t pin_x_bytes = 0, pin_y_bytes = 0;
     // f16 shadow copies of weight matrices for the prefill GEMM (option gemm_cache_weights):
     // key = (blocks pointer, n, k, qtype * 2 + order) -> device allocation of n*k halfs.
     std::map<std::tuple<const void *, int64_t, int64_t, int>, void *> w16_cache;

@@ -257,13 +257,19 @@ class QLinear {
         Device &dev = *w_.device();
         cq_ctx *ctx = dev.ctx();
         std::vector<float> y((size_t)(rows * w_.n));
+        if (!bias_.empty() && !bias_dev_) bias_dev_.reset(new Storage(Storage::from_slice(w_.device(), bias_)));
+        constexpr size_t kHostCall = (size_t(1) << 20) / sizeof(float);
+        if (x.size() <= kHostCall && y.size() <= kHostCall) {  // the whole call in the library, with one wait
+            check(ctx, cq_qlinear_host(ctx, w_.qtype, w_.order, actmode, x.data(), rows, k, w_.ptr(), w_.n, bias_dev_ ? bias_dev_->ptr() : nullptr, y.data()),
+                  "linear: failed to matmul");
+            return y;
+        }
         Device::Staged xs(dev, 4 * x.size()), ys(dev, 4 * y.size());
         check(ctx, cq_memcpy_h2d(ctx, xs.ptr(), x.data(), 4 * x.size()), "cuda: storage from slice");
         if (bias_.empty()) {
             check(ctx, cq_qmatmul(ctx, w_.qtype, w_.order, actmode, xs.ptr(), rows, k, k, w_.ptr(), w_.n, ys.ptr(), w_.n),
                   "matmul forward: failed to matmul");
         } else {  // BroadcastAdd (nn/linear.go:105-110) happens on the device, in the matmul's epilogue where its kernel has one
-            if (!bias_dev_) bias_dev_.reset(new Storage(Storage::from_slice(w_.device(), bias_)));
             check(ctx, cq_qlinear(ctx, w_.qtype, w_.order, actmode, xs.ptr(), rows, k, k, w_.ptr(), w_.n, bias_dev_->ptr(), ys.ptr(), w_.n),
                   "linear: failed to matmul");
         }

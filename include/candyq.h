@@ -212,12 +212,16 @@ cq_status cq_qlinear(cq_ctx *ctx, int qtype, int order, int actmode, const float
 
 /* Same product with HOST activations and HOST result: copies x up, runs cq_qmatmul, copies
  * y back and waits.  Weights stay resident on the device (they are the layer's state).
- * x_host / y_host should be pinned (cq_malloc_host) for full copy speed.  With at most eight rows and a
- * pinned y_host of up to host_zero_copy bytes (option, default 256 KiB; 0 turns it off) the kernel stores the
- * result into y_host directly and nothing is copied back; the bits are the same either way. */
+ * Any host memory will do; buffers that are not page-locked (cq_malloc_host) pass through blocks of the context that are, up
+ * to a megabyte each.  With at most eight rows and a result of up to host_zero_copy bytes (option, default 256 KiB; 0 turns it
+ * off) the kernel stores the result into page-locked memory directly and nothing is copied back; the bits are the same either way. */
 cq_status cq_qmatmul_host(cq_ctx *ctx, int qtype, int order, int actmode, const float *x_host,
                           int64_t m, int64_t k, const void *w_blocks_dev, int64_t n,
                           float *y_host);
+/* cq_qlinear with HOST activations and HOST result; bias_dev may be NULL. */
+cq_status cq_qlinear_host(cq_ctx *ctx, int qtype, int order, int actmode, const float *x_host,
+                          int64_t m, int64_t k, const void *w_blocks_dev, int64_t n,
+                          const float *bias_dev, float *y_host);
 
 /* Same product as cq_qmatmul(..., CQ_ACT_Q8_1, ...) for m <= 8, for callers that cannot let
  * the library allocate: hosts that gave all device memory to their own arena at start-up, or

@@ -14,6 +14,8 @@
 
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace {
@@ -535,204 +537,205 @@ __global__ void __launch_bounds__(128) attn_partial_gqa_kernel(const float *__re
     }
 }
 
-// Split-context grouped-query decode attention, hd == 128, G = nq/nkv <= 8.  One CTA per
-// (split of the context, kv head, sequence) walks its keys 64 at a time with a running softmax
-// and serves all G query heads of the group from one pass over K and V:
-//   load    64 keys and values into shared memory with 16-byte async copies (K rows padded to
-//           132 floats so that lane = key reads are conflict-free);
-//   scores  warp = quarter of the 128 dims, lane = keys (lane, lane+32): 2 x 8 accumulators,
-//           ten 16-byte shared loads per 64 FMAs; the four dim-quarters are summed through
-//           shared memory;
-//   softmax warp w owns heads 2w, 2w+1: running max and sum in registers, numerators and the
-//           rescaling factor to shared memory;
-//   values  warp = quarter of the 64 keys, lane = four dims: 8 x 4 accumulators kept in
-//           registers across the whole split, three 16-byte shared loads per 32 FMAs.
+// Split-context grouped-query decode attention, hd == 128, G = nq/nkv <= 8.  One CTA per (split of the context, kv head,
+// sequence), and each of its four warps by itself: no barrier until the end, K and V go from memory to registers.
+// A warp takes eight keys at a time:
+//   scores  eight lanes a key, two keys a lane: lane 8 s + c has values 4 c + 32 j .. + 3 of keys s and 4 + s; q comes from shared
+//           memory once for both; a butterfly over eight lanes leaves each with one head's score of its two keys
+//   softmax running maximum, sum and factor of a head in its lanes; p passes through the warp's 256 bytes of shared memory
+//   values  lane = four dims of all keys, pairs of heads per instruction
+// The next eight keys' K is in flight during softmax and values (in registers), V two rounds ahead (in the warp's own shared memory,
+// every lane its own dims): 8 to 12 KB a warp, sixteen warps an SM.
+// Bound: HBM (f32 caches, read once for all G heads).  The kernel before this one staged K and V in shared memory for the four
+// warps together, and read q and p from there, the same words for every lane: 2200 cycles of shared-memory bandwidth and three
+// barriers per 64 keys.  64 / 8 heads, 32 sequences x 2048 keys, us: before 140, now 108, floor 82;
+// 2 x 64 / 8 heads x 16384 72 -> 61, one sequence of 2048 keys 11.7 -> 12.4.
 // Writes (max, sum, acc[128]) per (head, split) in the layout the combine kernel reads.
-constexpr int kAttn2Keys = 64;
-constexpr int kAttn2KStride = 132;
-constexpr size_t kAttn2Smem = (size_t)kAttn2Keys * kAttn2KStride * 4 + (size_t)kAttn2Keys * 128 * 4  // K, V
-                              + 8 * 128 * 4                                                          // q
-                              + 4 * 8 * kAttn2Keys * 4                                               // score partials [warp][head][key]
-                              + kAttn2Keys * 8 * 4 + 64;                                             // numerators [key][head], factors
+constexpr int kAttn2Keys = 32;  // keys that a CTA takes per round: splits are multiples of it
+constexpr int kAttn2Stages = 3; // rounds of V in shared memory
+constexpr size_t kAttn2Smem = (size_t)4 * kAttn2Stages * 8 * 128 * 4;  // [warp][round][key][dim]; at the end the warps' sums
 template <bool ROPE>
-__global__ void __launch_bounds__(128) attn_split_gqa_kernel(const float *__restrict__ qkv, int nq, int nkv, const int *__restrict__ pos_dev,
-                                                           const float *kc, const float *vc, int max_ctx, float scale,
-                                                           float *__restrict__ part, int nsplits, int keys_per_split,
-                                                           const float *__restrict__ cos_t, const float *__restrict__ sin_t, float *kc_w,
-                                                           float *vc_w, int *err) {
+__global__ void __launch_bounds__(128, 4) attn_split_gqa_kernel(const float *__restrict__ qkv, int nq, int nkv, const int *__restrict__ pos_dev,
+                                                              const float *kc, const float *vc, int max_ctx, float scale, float *__restrict__ part,
+                                                              int nsplits, const float *__restrict__ cos_t, const float *__restrict__ sin_t, float *kc_w,
+                                                              float *vc_w, int *err) {
     constexpr int hd = 128;
-    extern __shared__ __align__(16) uint8_t attn_smem[];
-    float *Ks = reinterpret_cast<float *>(attn_smem);
-    float *Vs = Ks + kAttn2Keys * kAttn2KStride;
-    float *q_s = Vs + kAttn2Keys * hd;
-    float *sp_s = q_s + 8 * hd;                  // [4][8][64]
-    float *p_s = sp_s + 4 * 8 * kAttn2Keys;      // [64][8]
-    float *alpha_s = p_s + kAttn2Keys * 8;       // [8]
+    constexpr float kLow = -3.402823466e38f;
+    extern __shared__ __align__(16) float attn_smem[];
+    float(*acc_s)[8][hd] = reinterpret_cast<float(*)[8][hd]>(attn_smem);
+    __shared__ __align__(16) float q_s[8][hd], p_s[4][8][8], f_s[4][8];
+    __shared__ float m_s[4][8], l_s[4][8];
     pdl_launch_dependents();
     pdl_wait_prior();
     const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
     const int G = nq / nkv;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nkeys = checked_pos(pos_dev, max_ctx, err) + 1;
+    // equal shares of the keys that there are, in whole rounds
+    const int keys_per_split = ((nkeys + nsplits - 1) / nsplits + kAttn2Keys - 1) / kAttn2Keys * kAttn2Keys;
     const int t_begin = split * keys_per_split;
     const int t_end = min(t_begin + keys_per_split, nkeys);
     const int stride = hd + 2;
-    if (t_begin >= t_end) {  // split beyond the current length: neutral element
+    if (t_begin >= t_end) {  // nothing left for this split: neutral element
         for (int g = 0; g < G; ++g) {
             float *out = part + (((int64_t)b * nq + kvh * G + g) * nsplits + split) * stride;
-            if (tid == 0) out[0] = -3.402823466e38f, out[1] = 0.0f;
+            if (tid == 0) out[0] = kLow, out[1] = 0.0f;
             out[2 + tid] = 0.0f;
         }
         return;
     }
     const int row = (nq + 2 * nkv) * hd;
     const int64_t kv_stride = (int64_t)nkv * hd;
-    const float *kbase = kc + ((int64_t)b * max_ctx) * kv_stride + kvh * hd;
-    const float *vbase = vc + ((int64_t)b * max_ctx) * kv_stride + kvh * hd;
-    // q of the group's heads (rotated here when the rotary step is fused in: cos_t given)
+    const int slot = lane >> 3, c = lane & 7;  // of the scores
+    const float *kbase = kc + ((int64_t)b * max_ctx) * kv_stride + kvh * hd + 4 * c;
+    const float *vbase = vc + ((int64_t)b * max_ctx) * kv_stride + kvh * hd + 4 * lane;
+    uint64_t acc[4][4];  // [pair of heads][dim]
+#pragma unroll
+    for (int g = 0; g < 4; ++g)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[g][i] = 0;
+    // Rows past the end repeat the last one (their p is 0, and their V is made 0).  The newest key is not in the cache yet where the
+    // rotary step is fused in: rotated k / plain v come from qkv, and the lanes that own it (the only ones of its kv head and
+    // sequence) store them to the cache.
+    const float *k_new = qkv + (int64_t)b * row + (nq + kvh) * hd, *v_new = k_new + (int64_t)nkv * hd;
+    const int64_t newest = ((int64_t)b * max_ctx + nkeys - 1) * kv_stride + kvh * hd;
+    auto fetch_k = [&](int t, float4(&r)[2][4]) {
+#pragma unroll
+        for (int kk = 0; kk < 2; ++kk) {
+            const int at = t + 4 * kk + slot, key = min(at, t_end - 1);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (ROPE && key == nkeys - 1) {
+                    const int d = 4 * c + 32 * j;
+                    r[kk][j] = make_float4(rope_elem(k_new, d, hd, cos_t, sin_t, key), rope_elem(k_new, d + 1, hd, cos_t, sin_t, key),
+                                           rope_elem(k_new, d + 2, hd, cos_t, sin_t, key), rope_elem(k_new, d + 3, hd, cos_t, sin_t, key));
+                    if (at == key) *reinterpret_cast<float4 *>(kc_w + newest + d) = r[kk][j];
+                } else {
+                    r[kk][j] = __ldcs(reinterpret_cast<const float4 *>(kbase + (int64_t)key * kv_stride + 32 * j));
+                }
+            }
+        }
+    };
+    float *v_ring = attn_smem + (size_t)warp * kAttn2Stages * 8 * hd + 4 * lane;
+    auto fetch_v = [&](int t, int stage) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            float *dst = v_ring + (stage * 8 + i) * hd;
+            if (ROPE && t + i == nkeys - 1 && t + i < t_end) {
+                const float4 v = *reinterpret_cast<const float4 *>(v_new + 4 * lane);
+                *reinterpret_cast<float4 *>(dst) = v;
+                *reinterpret_cast<float4 *>(vc_w + newest + 4 * lane) = v;
+            } else {  // (no bytes past the end: zeros)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                             "l"(vbase + (int64_t)min(t + i, t_end - 1) * kv_stride), "r"(t + i < t_end ? 16 : 0)
+                             : "memory");
+            }
+        }
+    };
+    auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
+    float m_run = kLow, l_run = 0.0f;  // of head c: its maximum so far, and this lane's part of its sum
+    float4 kr[2][4];
+    int t = t_begin + 8 * warp, stage = 0;
+    if (t < t_end) {
+        fetch_k(t, kr);
+        fetch_v(t, 0);
+    }
+    commit();
+    if (t + 32 < t_end) fetch_v(t + 32, 1);
+    commit();
+    // q of the group's heads (rotated here when the rotary step is fused in: cos_t given), while the first keys are on their way
     for (int i = tid; i < 8 * hd; i += 128) {
         const float *qh = qkv + (int64_t)b * row + (kvh * G + i / hd) * hd;
-        q_s[i] = (i / hd) < G ? (ROPE ? rope_elem(qh, i % hd, hd, cos_t, sin_t, nkeys - 1) : qh[i % hd]) : 0.0f;
+        q_s[i / hd][i % hd] = (i / hd) < G ? (ROPE ? rope_elem(qh, i % hd, hd, cos_t, sin_t, nkeys - 1) : qh[i % hd]) : 0.0f;
     }
-
-    float m_run[2] = {-3.402823466e38f, -3.402823466e38f}, l_run[2] = {0.0f, 0.0f};  // heads 2*warp, 2*warp+1 (lane-uniform)
-    float acc[8][4];
+    __syncthreads();
+    for (; t < t_end; t += 32) {
+        if (t + 64 < t_end) fetch_v(t + 64, stage == 0 ? 2 : stage - 1);
+        commit();
+        float s[2][8];
 #pragma unroll
-    for (int g = 0; g < 8; ++g)
+        for (int g = 0; g < 8; ++g) {
+            uint64_t x0[2] = {0, 0}, x1[2] = {0, 0};  // two chains a key
 #pragma unroll
-        for (int i = 0; i < 4; ++i) acc[g][i] = 0.0f;
-
-    // 64 rows of K (or V) starting at key t0 into shared memory, as one async-copy group; rows past
-    // the end become zeros, so that no stale NaN reaches a product with a zero weight.  A warp copies
-    // one 512-byte row per instruction.
-    auto load_rows = [&](const float *base, float *dst, int dst_stride, int t0) {
-        const int cnt = min(kAttn2Keys, t_end - t0);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const int f = tid + 128 * j, r = f >> 5, c4 = f & 31;
-            float *d = dst + r * dst_stride + 4 * c4;
-            if (ROPE && r < cnt && t0 + r == nkeys - 1) {
-                // the newest key is not in the cache yet: rotated k / plain v come from qkv, and this CTA
-                // (the only one of its kv head and sequence that sees this row) stores them to the cache
-                const bool is_k = base == kbase;
-                const float *src = qkv + (int64_t)b * row + (nq + (is_k ? 0 : nkv) + kvh) * hd;
-                float4 v4;
-                if (is_k) v4 = make_float4(rope_elem(src, 4 * c4, hd, cos_t, sin_t, t0 + r), rope_elem(src, 4 * c4 + 1, hd, cos_t, sin_t, t0 + r),
-                                           rope_elem(src, 4 * c4 + 2, hd, cos_t, sin_t, t0 + r), rope_elem(src, 4 * c4 + 3, hd, cos_t, sin_t, t0 + r));
-                else v4 = *reinterpret_cast<const float4 *>(src + 4 * c4);
-                *reinterpret_cast<float4 *>(d) = v4;
-                *reinterpret_cast<float4 *>((is_k ? kc_w : vc_w) + ((int64_t)b * max_ctx + t0 + r) * kv_stride + kvh * hd + 4 * c4) = v4;
-            } else if (r < cnt) {
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(d)),
-                             "l"(base + (int64_t)(t0 + r) * kv_stride + 4 * c4)
-                             : "memory");
-            } else {
-                *reinterpret_cast<float4 *>(d) = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int j = 0; j < 4; ++j) {
+                const ulonglong2 q = *reinterpret_cast<const ulonglong2 *>(&q_s[g][4 * c + 32 * j]);
+                x0[j & 1] = fma2(q.y, pack2(kr[0][j].z, kr[0][j].w), fma2(q.x, pack2(kr[0][j].x, kr[0][j].y), x0[j & 1]));
+                x1[j & 1] = fma2(q.y, pack2(kr[1][j].z, kr[1][j].w), fma2(q.x, pack2(kr[1][j].x, kr[1][j].y), x1[j & 1]));
             }
+            float lo, hi;
+            unpack2(add2(x0[0], x0[1]), lo, hi), s[0][g] = lo + hi;
+            unpack2(add2(x1[0], x1[1]), lo, hi), s[1][g] = lo + hi;
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    // Software pipeline over two buffers: K of the next chunk streams in during this chunk's softmax
-    // and value pass, V of the next chunk during the next chunk's scores.
-    load_rows(kbase, Ks, kAttn2KStride, t_begin);
-    load_rows(vbase, Vs, hd, t_begin);
-    for (int t0 = t_begin; t0 < t_end; t0 += kAttn2Keys) {
-        const int cnt = min(kAttn2Keys, t_end - t0);
-        const bool more = t0 + kAttn2Keys < t_end;
-        asm volatile("cp.async.wait_group 1;" ::: "memory");  // K of this chunk has landed (V may still be in flight)
-        __syncthreads();
-        // ---- scores: this warp's 32 dims, keys lane and lane+32, all eight heads --------------------
-        {
-            float s[2][8];
+        if (t + 32 < t_end) fetch_k(t + 32, kr);
 #pragma unroll
-            for (int g = 0; g < 8; ++g) s[0][g] = 0.0f, s[1][g] = 0.0f;
-            const float *k0 = Ks + lane * kAttn2KStride + 32 * warp, *k1 = k0 + 32 * kAttn2KStride;
-            const float *qw = q_s + 32 * warp;
+        for (int o = 4; o > 0; o >>= 1)
 #pragma unroll
-            for (int d4 = 0; d4 < 8; ++d4) {
-                const float4 a = *reinterpret_cast<const float4 *>(k0 + 4 * d4), c = *reinterpret_cast<const float4 *>(k1 + 4 * d4);
+            for (int kk = 0; kk < 2; ++kk)
 #pragma unroll
-                for (int g = 0; g < 8; ++g) {
-                    const float4 q = *reinterpret_cast<const float4 *>(qw + g * hd + 4 * d4);
-                    s[0][g] = fmaf(q.x, a.x, fmaf(q.y, a.y, fmaf(q.z, a.z, fmaf(q.w, a.w, s[0][g]))));
-                    s[1][g] = fmaf(q.x, c.x, fmaf(q.y, c.y, fmaf(q.z, c.z, fmaf(q.w, c.w, s[1][g]))));
+                for (int j = 0; j < o; ++j) {
+                    const bool up = (lane & o) != 0;
+                    const float give = up ? s[kk][j] : s[kk][j + o], keep = up ? s[kk][j + o] : s[kk][j];
+                    s[kk][j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
                 }
-            }
+        // lane 8 s + c: head c, keys t + s and t + 4 + s
+        const bool live0 = t + slot < t_end, live1 = t + 4 + slot < t_end;
+        const float sc0 = live0 ? s[0][0] * scale : kLow, sc1 = live1 ? s[1][0] * scale : kLow;
+        float m_new = fmaxf(sc0, sc1);
+        m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 8));
+        m_new = fmaxf(m_run, fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 16)));
+        const float p0 = live0 ? expf(sc0 - m_new) : 0.0f, p1 = live1 ? expf(sc1 - m_new) : 0.0f;
+        const bool moved = __any_sync(0xffffffffu, m_new != m_run);
+        const float f = moved ? expf(m_run - m_new) : 1.0f;  // 0 on the first keys
+        l_run = fmaf(l_run, f, p0 + p1);
+        m_run = m_new;
+        __syncwarp();  // the round before has read its p
+        (&p_s[warp][0][0])[lane] = p0;
+        (&p_s[warp][0][0])[32 + lane] = p1;
+        if (moved && lane < 8) f_s[warp][lane] = f;
+        __syncwarp();
+        if (moved) {
+            const ulonglong2 f0 = *reinterpret_cast<const ulonglong2 *>(&f_s[warp][0]), f1 = *reinterpret_cast<const ulonglong2 *>(&f_s[warp][4]);
 #pragma unroll
-            for (int g = 0; g < 8; ++g) {
-                sp_s[(warp * 8 + g) * kAttn2Keys + lane] = s[0][g];
-                sp_s[(warp * 8 + g) * kAttn2Keys + lane + 32] = s[1][g];
+            for (int i = 0; i < 4; ++i) acc[0][i] = mul2(acc[0][i], f0.x), acc[1][i] = mul2(acc[1][i], f0.y), acc[2][i] = mul2(acc[2][i], f1.x), acc[3][i] = mul2(acc[3][i], f1.y);
+        }
+        asm volatile("cp.async.wait_group 2;" ::: "memory");
+        const float *v_now = v_ring + stage * 8 * hd;
+        stage = stage == kAttn2Stages - 1 ? 0 : stage + 1;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float4 vi = *reinterpret_cast<const float4 *>(v_now + i * hd);
+            const ulonglong2 pa = *reinterpret_cast<const ulonglong2 *>(&p_s[warp][i][0]), pb = *reinterpret_cast<const ulonglong2 *>(&p_s[warp][i][4]);
+            const uint64_t v[4] = {dup2(vi.x), dup2(vi.y), dup2(vi.z), dup2(vi.w)};
+#pragma unroll
+            for (int d = 0; d < 4; ++d) {
+                acc[0][d] = fma2(pa.x, v[d], acc[0][d]);
+                acc[1][d] = fma2(pa.y, v[d], acc[1][d]);
+                acc[2][d] = fma2(pb.x, v[d], acc[2][d]);
+                acc[3][d] = fma2(pb.y, v[d], acc[3][d]);
             }
         }
-        __syncthreads();
-        if (more) load_rows(kbase, Ks, kAttn2KStride, t0 + kAttn2Keys);  // K buffer is free
-        else asm volatile("cp.async.commit_group;" ::: "memory");         // keep the group count uniform
-        // ---- running softmax: warp w owns heads 2w and 2w+1 ------------------------------------------
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-            const int g = 2 * warp + hh;
-            float sc[2];
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                const int t = lane + 32 * half;
-                const float v = (sp_s[(0 * 8 + g) * kAttn2Keys + t] + sp_s[(1 * 8 + g) * kAttn2Keys + t]) +
-                                (sp_s[(2 * 8 + g) * kAttn2Keys + t] + sp_s[(3 * 8 + g) * kAttn2Keys + t]);
-                sc[half] = t < cnt ? v * scale : -3.402823466e38f;
-            }
-            const float m_new = fmaxf(m_run[hh], warp_max(fmaxf(sc[0], sc[1])));
-            const float e0 = lane < cnt ? expf(sc[0] - m_new) : 0.0f;
-            const float e1 = lane + 32 < cnt ? expf(sc[1] - m_new) : 0.0f;
-            const float a = expf(m_run[hh] - m_new);  // 0 on the first chunk
-            l_run[hh] = l_run[hh] * a + warp_sum(e0 + e1);
-            m_run[hh] = m_new;
-            p_s[lane * 8 + g] = e0;
-            p_s[(lane + 32) * 8 + g] = e1;
-            if (lane == 0) alpha_s[g] = a;
-        }
-        asm volatile("cp.async.wait_group 1;" ::: "memory");  // V of this chunk has landed (the next K may still be in flight)
-        __syncthreads();
-        // ---- values: this warp's 16 keys, dims 4*lane .. 4*lane+3, all eight heads ---------------------
-        {
-            const float4 a0 = *reinterpret_cast<const float4 *>(alpha_s), a1 = *reinterpret_cast<const float4 *>(alpha_s + 4);
-            const float al[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-#pragma unroll
-            for (int g = 0; g < 8; ++g)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) acc[g][i] *= al[g];
-#pragma unroll 4
-            for (int tt = 0; tt < 16; ++tt) {
-                const int t = 16 * warp + tt;
-                const float4 v = *reinterpret_cast<const float4 *>(Vs + t * hd + 4 * lane);
-                const float4 p0 = *reinterpret_cast<const float4 *>(p_s + t * 8), p1 = *reinterpret_cast<const float4 *>(p_s + t * 8 + 4);
-                const float pw[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
-#pragma unroll
-                for (int g = 0; g < 8; ++g) {
-                    acc[g][0] = fmaf(pw[g], v.x, acc[g][0]);
-                    acc[g][1] = fmaf(pw[g], v.y, acc[g][1]);
-                    acc[g][2] = fmaf(pw[g], v.z, acc[g][2]);
-                    acc[g][3] = fmaf(pw[g], v.w, acc[g][3]);
-                }
-            }
-        }
-        __syncthreads();
-        if (more) load_rows(vbase, Vs, hd, t0 + kAttn2Keys);  // V buffer is free
-        else asm volatile("cp.async.commit_group;" ::: "memory");
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    // ---- the four key-quarters' accumulators are summed through shared memory (K region) ---------
-    __syncthreads();
-    float *red = Ks;  // [4][8][128]
+    l_run += __shfl_xor_sync(0xffffffffu, l_run, 8);
+    l_run += __shfl_xor_sync(0xffffffffu, l_run, 16);
+    __syncthreads();  // everybody is done with the rings
+    // ---- the four warps' parts, brought to one maximum ----------------------------------------
+    if (lane < 8) m_s[warp][lane] = m_run, l_s[warp][lane] = l_run;
 #pragma unroll
-    for (int g = 0; g < 8; ++g) *reinterpret_cast<float4 *>(red + (warp * 8 + g) * hd + 4 * lane) = make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]);
-    if (lane == 0) {
-        alpha_s[2 * warp] = m_run[0], alpha_s[2 * warp + 1] = m_run[1];
-        p_s[2 * warp] = l_run[0], p_s[2 * warp + 1] = l_run[1];
+    for (int g = 0; g < 4; ++g) {
+        float4 lo, hi;
+        unpack2(acc[g][0], lo.x, hi.x), unpack2(acc[g][1], lo.y, hi.y), unpack2(acc[g][2], lo.z, hi.z), unpack2(acc[g][3], lo.w, hi.w);
+        *reinterpret_cast<float4 *>(&acc_s[warp][2 * g][4 * lane]) = lo, *reinterpret_cast<float4 *>(&acc_s[warp][2 * g + 1][4 * lane]) = hi;
     }
     __syncthreads();
-    for (int g = 0; g < G; ++g) {
+#pragma unroll
+    for (int g = 0; g < 8; ++g) {
+        if (g >= G) break;
         float *out = part + (((int64_t)b * nq + kvh * G + g) * nsplits + split) * stride;
-        out[2 + tid] = (red[(0 * 8 + g) * hd + tid] + red[(1 * 8 + g) * hd + tid]) + (red[(2 * 8 + g) * hd + tid] + red[(3 * 8 + g) * hd + tid]);
-        if (tid == 0) out[0] = alpha_s[g], out[1] = p_s[g];
+        const float m = fmaxf(fmaxf(m_s[0][g], m_s[1][g]), fmaxf(m_s[2][g], m_s[3][g]));
+        const float f0 = expf(m_s[0][g] - m), f1 = expf(m_s[1][g] - m), f2 = expf(m_s[2][g] - m), f3 = expf(m_s[3][g] - m);
+        out[2 + tid] = (f0 * acc_s[0][g][tid] + f1 * acc_s[1][g][tid]) + (f2 * acc_s[2][g][tid] + f3 * acc_s[3][g][tid]);
+        if (tid == 0) out[0] = m, out[1] = (f0 * l_s[0][g] + f1 * l_s[1][g]) + (f2 * l_s[2][g] + f3 * l_s[3][g]);
     }
 }
 
@@ -1091,14 +1094,16 @@ cq_status attention_impl(cq_ctx *ctx, float *qkv_dev, int64_t batch, int n_q_hea
         return CQ_OK;
     }
     if (split_route) {
-        // splits of the context sized so that about four CTAs per SM exist, never under 64 keys each
-        const int64_t pairs = (int64_t)n_kv_heads * batch;
-        int64_t want = ((int64_t)ctx->sm_count * 4 + pairs - 1) / pairs;
-        const int max_splits = (max_ctx + kAttn2Keys - 1) / kAttn2Keys;
-        if (want > max_splits) want = max_splits;
-        if (want < 1) want = 1;
-        const int keys_per_split = (int)(((max_ctx + want - 1) / want + kAttn2Keys - 1) / kAttn2Keys) * kAttn2Keys;
-        nchunks = (max_ctx + keys_per_split - 1) / keys_per_split;
+        // Splits of the keys: what a round of CTAs (four per SM) takes at the longest context, its keys and about 96 keys' worth of
+        // start and end, times the rounds, and two keys' worth per split for combining.  (us with 1, 2, 4, 8, 16, 32, 64 splits: 32
+        // sequences x 8 kv heads x 2048 keys 177, 108, 103, 111, 129, 163, 235; 4 x 8 x 2048 68, 37, 34, 22, 18.5, 21, 26; 1 x 8 x 2048
+        // 67, 36, 22, 14.5, 13.3, 12.4, 13.4; 2 x 8 x 16384 492, 254, 134, 114, 69, 61, 66; 1 x 8 x 128 9.4, 7.7, 6.7.)
+        const int64_t pairs = (int64_t)n_kv_heads * batch, slots = (int64_t)ctx->sm_count * 4;
+        int64_t best = INT64_MAX;
+        for (int i = 1, most = std::min(nchunks, 64); i <= most; ++i) {  // (a chunk of scratch is 32 keys)
+            const int64_t cost = (pairs * i + slots - 1) / slots * ((max_ctx + i - 1) / i + 96) + 2 * i;
+            if (cost < best) best = cost, nchunks = i;
+        }
         static thread_local int configured = -1;
         if (configured != ctx->device) {
             CQ_CUDA(ctx, cudaFuncSetAttribute(attn_split_gqa_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAttn2Smem));
@@ -1117,11 +1122,11 @@ cq_status attention_impl(cq_ctx *ctx, float *qkv_dev, int64_t batch, int n_q_hea
         cfg.numAttrs = ctx->tune.pdl ? 1 : 0;
         if (cos_dev)
             CQ_CUDA(ctx, cudaLaunchKernelEx(&cfg, attn_split_gqa_kernel<true>, (const float *)qkv_dev, n_q_heads, n_kv_heads, pos_dev, (const float *)k_cache_dev,
-                                        (const float *)v_cache_dev, max_ctx, scale, scratch_dev, nchunks, keys_per_split, cos_dev, sin_dev,
+                                        (const float *)v_cache_dev, max_ctx, scale, scratch_dev, nchunks, cos_dev, sin_dev,
                                         k_cache_dev, v_cache_dev, ctx->dev_err_devptr));
         else
             CQ_CUDA(ctx, cudaLaunchKernelEx(&cfg, attn_split_gqa_kernel<false>, (const float *)qkv_dev, n_q_heads, n_kv_heads, pos_dev, (const float *)k_cache_dev,
-                                        (const float *)v_cache_dev, max_ctx, scale, scratch_dev, nchunks, keys_per_split, cos_dev, sin_dev,
+                                        (const float *)v_cache_dev, max_ctx, scale, scratch_dev, nchunks, cos_dev, sin_dev,
                                         k_cache_dev, v_cache_dev, ctx->dev_err_devptr));
         s = CQ_OK;
     } else if (gqa_chunk_route)

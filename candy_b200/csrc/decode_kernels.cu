@@ -53,21 +53,47 @@ __global__ void __launch_bounds__(1024) rmsnorm_kernel(float *__restrict__ x, co
     float *xr = x + (int64_t)blockIdx.x * cols;
     const float *dr = ADD ? delta + (int64_t)blockIdx.x * cols : nullptr;
     float *yr = y + (int64_t)blockIdx.x * cols;
-    float ss = 0.0f;
-    for (int c = threadIdx.x; c < cols; c += blockDim.x) {
-        float v = xr[c];
-        if (ADD) {
-            v += dr[c];
-            xr[c] = v;
+    constexpr int HELD = 8;  // values a thread keeps: all loads of a row in flight at once, and none read twice (rows of 4096 x 128 6.9 -> us)
+    const bool held = cols <= HELD * (int)blockDim.x;
+    float v[HELD], d[HELD], w[HELD], ss = 0.0f;
+    if (held) {
+#pragma unroll
+        for (int i = 0; i < HELD; ++i) {
+            const int c = threadIdx.x + i * blockDim.x;
+            v[i] = c < cols ? xr[c] : 0.0f;
+            d[i] = ADD && c < cols ? dr[c] : 0.0f;
+            w[i] = alpha && c < cols ? alpha[c] : 0.0f;
         }
-        ss = fmaf(v, v, ss);
+#pragma unroll
+        for (int i = 0; i < HELD; ++i) {
+            const int c = threadIdx.x + i * blockDim.x;
+            if (ADD && c < cols) xr[c] = v[i] += d[i];
+            ss = fmaf(v[i], v[i], ss);
+        }
+    } else {
+        for (int c = threadIdx.x; c < cols; c += blockDim.x) {
+            float t = xr[c];
+            if (ADD) {
+                t += dr[c];
+                xr[c] = t;
+            }
+            ss = fmaf(t, t, ss);
+        }
     }
     ss = block_sum(ss, sh);
     const float mean = ss / (float)cols;
     const float scale = 1.0f / sqrtf(mean + eps);
-    for (int c = threadIdx.x; c < cols; c += blockDim.x) {
-        const float v = xr[c];  // own writes above are visible to the same thread
-        yr[c] = alpha ? scale * v * alpha[c] : scale * v;
+    if (held) {
+#pragma unroll
+        for (int i = 0; i < HELD; ++i) {
+            const int c = threadIdx.x + i * blockDim.x;
+            if (c < cols) yr[c] = alpha ? scale * v[i] * w[i] : scale * v[i];
+        }
+    } else {
+        for (int c = threadIdx.x; c < cols; c += blockDim.x) {
+            const float t = xr[c];  // own writes above are visible to the same thread
+            yr[c] = alpha ? scale * t * alpha[c] : scale * t;
+        }
     }
 }
 
@@ -147,7 +173,7 @@ __device__ __forceinline__ uint16_t to16(float v) {
 template <bool BF16>
 __global__ void __launch_bounds__(256) rope_prefill_kernel(const float *__restrict__ qkv, int T, int nq, int nkv, int hd, const float *__restrict__ cos_t,
                                                          const float *__restrict__ sin_t, int pos0, float *__restrict__ kc, float *__restrict__ vc,
-                                                         uint16_t *__restrict__ q16, uint16_t *__restrict__ k16, uint16_t *__restrict__ v16) {
+                                                         uint16_t *__restrict__ q16, uint16_t *__restrict__ k16, uint16_t *__restrict__ v16, int vec) {
     pdl_launch_dependents();
     pdl_wait_prior();
     const int t = blockIdx.y;
@@ -157,6 +183,34 @@ __global__ void __launch_bounds__(256) rope_prefill_kernel(const float *__restri
     const float *base = qkv + (int64_t)t * row;
     const int npairs = (nq + nkv) * half;
     const int64_t cache_row = (int64_t)pos * (int64_t)(nkv * hd);
+    if (vec) {  // four pairs, or four values of v, a thread
+        auto pack4 = [](float x, float y, float z, float w) {
+            return make_uint2(to16<BF16>(x) | (uint32_t)to16<BF16>(y) << 16, to16<BF16>(z) | (uint32_t)to16<BF16>(w) << 16);
+        };
+        const int i = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+        if (i < npairs) {
+            const int head = i / half, d = i - head * half;
+            const float *p = base + head * hd + d;
+            const float4 c = *reinterpret_cast<const float4 *>(cos_t + (int64_t)pos * half + d), s = *reinterpret_cast<const float4 *>(sin_t + (int64_t)pos * half + d);
+            const float4 a = *reinterpret_cast<const float4 *>(p), bb = *reinterpret_cast<const float4 *>(p + half);
+            const float4 r1 = make_float4(a.x * c.x - bb.x * s.x, a.y * c.y - bb.y * s.y, a.z * c.z - bb.z * s.z, a.w * c.w - bb.w * s.w);
+            const float4 r2 = make_float4(a.x * s.x + bb.x * c.x, a.y * s.y + bb.y * c.y, a.z * s.z + bb.z * c.z, a.w * s.w + bb.w * c.w);
+            uint16_t *dst = head < nq ? q16 + ((int64_t)t * nq + head) * hd + d : k16 + ((int64_t)t * nkv + (head - nq)) * hd + d;
+            *reinterpret_cast<uint2 *>(dst) = pack4(r1.x, r1.y, r1.z, r1.w);
+            *reinterpret_cast<uint2 *>(dst + half) = pack4(r2.x, r2.y, r2.z, r2.w);
+            if (head >= nq) {
+                float *kdst = kc + cache_row + (head - nq) * hd + d;
+                *reinterpret_cast<float4 *>(kdst) = r1;
+                *reinterpret_cast<float4 *>(kdst + half) = r2;
+            }
+        } else if (i < npairs + nkv * hd) {
+            const int j = i - npairs;
+            const float4 v = *reinterpret_cast<const float4 *>(base + (nq + nkv) * hd + j);
+            *reinterpret_cast<float4 *>(vc + cache_row + j) = v;
+            *reinterpret_cast<uint2 *>(v16 + (int64_t)t * nkv * hd + j) = pack4(v.x, v.y, v.z, v.w);
+        }
+        return;
+    }
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npairs + nkv * hd; i += gridDim.x * blockDim.x) {
         if (i < npairs) {
             const int head = i / half, d = i - head * half;  // heads 0..nq-1 are q, then nkv k heads
@@ -196,8 +250,14 @@ template <bool BF16>
 __global__ void __launch_bounds__(256) cast16_to_f32_kernel(const uint16_t *__restrict__ src, int64_t n, float *__restrict__ dst) {
     pdl_launch_dependents();
     pdl_wait_prior();
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        dst[i] = BF16 ? __bfloat162float(__ushort_as_bfloat16(src[i])) : __half2float(__ushort_as_half(src[i]));
+    const int64_t step = (int64_t)gridDim.x * blockDim.x, first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    auto value = [](uint32_t v) { return BF16 ? __uint_as_float(v << 16) : __half2float(__ushort_as_half((unsigned short)v)); };
+    const int64_t whole = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0 ? n / 4 : 0;  // four values a thread
+    for (int64_t i = first; i < whole; i += step) {
+        const uint2 v = reinterpret_cast<const uint2 *>(src)[i];
+        reinterpret_cast<float4 *>(dst)[i] = make_float4(value(v.x & 0xFFFFu), value(v.x >> 16), value(v.y & 0xFFFFu), value(v.y >> 16));
+    }
+    for (int64_t i = 4 * whole + first; i < n; i += step) dst[i] = value(src[i]);
 }
 
 constexpr int kAttnChunk = 32;    // keys per CTA: short chunks keep many CTAs in flight at small contexts
@@ -829,16 +889,27 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const float *__restrict__
     }
 }
 
-// The same on (gate, up) pairs: out[b][i] = silu(gu[b][2i]) * gu[b][2i + 1].
-__global__ void __launch_bounds__(256) silu_mul_pairs_kernel(const float *__restrict__ gu, int n, int64_t total, float *__restrict__ out,
+// The same on (gate, up) pairs: out[b][i] = silu(gu[b][2i]) * gu[b][2i + 1].  Two outputs a thread where the rows allow it.
+__device__ __forceinline__ float silu_mul(float g, float u) {
+    const double x = (double)g;
+    return (float)(x / (1.0 + exp(-x))) * u;
+}
+__global__ void __launch_bounds__(256) silu_mul_pairs_kernel(const float *__restrict__ gu, int n, int64_t rows, int vec, float *__restrict__ out,
                                                            int64_t ld_out) {
     pdl_launch_dependents();
     pdl_wait_prior();
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t b = i / n, c = i - b * n;
-        const float2 v = *reinterpret_cast<const float2 *>(gu + b * 2 * n + 2 * c);
-        const double g = (double)v.x;
-        out[b * ld_out + c] = (float)(g / (1.0 + exp(-g))) * v.y;
+    const int64_t c = ((int64_t)blockIdx.x * 256 + threadIdx.x) * (vec ? 2 : 1);
+    if (c >= n) return;
+    for (int64_t b = blockIdx.y; b < rows; b += gridDim.y) {
+        const float *src = gu + 2 * (b * n + c);
+        float *dst = out + b * ld_out + c;
+        if (vec) {
+            const float4 v = *reinterpret_cast<const float4 *>(src);
+            *reinterpret_cast<float2 *>(dst) = make_float2(silu_mul(v.x, v.y), silu_mul(v.z, v.w));
+        } else {
+            const float2 v = *reinterpret_cast<const float2 *>(src);
+            *dst = silu_mul(v.x, v.y);
+        }
     }
 }
 
@@ -912,7 +983,12 @@ __global__ void __launch_bounds__(256) embedding_kernel(const float *__restrict_
     const int b = blockIdx.x;
     int64_t id = ids[b];
     if (id >= vocab) id = vocab - 1;  // never read outside the table
-    for (int c = threadIdx.x; c < dim; c += blockDim.x) out[(int64_t)b * dim + c] = table[id * dim + c];
+    if (((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(out)) & 15) == 0 && dim % 4 == 0) {
+#pragma unroll 4
+        for (int c = threadIdx.x; c < dim / 4; c += blockDim.x) reinterpret_cast<float4 *>(out + (int64_t)b * dim)[c] = reinterpret_cast<const float4 *>(table + id * dim)[c];
+    } else {
+        for (int c = threadIdx.x; c < dim; c += blockDim.x) out[(int64_t)b * dim + c] = table[id * dim + c];
+    }
 }
 
 __global__ void add_int_kernel(int *p, int delta) {
@@ -1016,13 +1092,17 @@ cq_status cq_rope_prefill(cq_ctx *ctx, const float *qkv_dev, int64_t tokens, int
         return cq_fail(ctx, CQ_ERR_INVALID_ARG, "cq_rope_prefill: bad shape");
     if (pos0 < 0 || (int64_t)pos0 + tokens > max_ctx)
         return cq_fail(ctx, CQ_ERR_INVALID_ARG, "cq_rope_prefill: positions pos0 .. pos0 + tokens - 1 must lie inside [0, max_ctx)");
-    const int work = (n_q_heads + n_kv_heads) * head_dim / 2 + n_kv_heads * head_dim;
+    int vec = head_dim % 8 == 0;
+    for (const void *q : {(const void *)qkv_dev, (const void *)cos_dev, (const void *)sin_dev, (const void *)k_cache_dev, (const void *)v_cache_dev, (const void *)q16_dev,
+                          (const void *)k16_dev, (const void *)v16_dev})
+        if (reinterpret_cast<uintptr_t>(q) & 15) vec = 0;
+    const int work = ((n_q_heads + n_kv_heads) * head_dim / 2 + n_kv_heads * head_dim) / (vec ? 4 : 1);
     const dim3 grid((unsigned)((work + 255) / 256), (unsigned)tokens);
     if (is_bf16)
         return launch_pdl(ctx, rope_prefill_kernel<true>, grid, dim3(256), qkv_dev, (int)tokens, n_q_heads, n_kv_heads, head_dim, cos_dev, sin_dev, pos0,
-                          k_cache_dev, v_cache_dev, static_cast<uint16_t *>(q16_dev), static_cast<uint16_t *>(k16_dev), static_cast<uint16_t *>(v16_dev));
+                          k_cache_dev, v_cache_dev, static_cast<uint16_t *>(q16_dev), static_cast<uint16_t *>(k16_dev), static_cast<uint16_t *>(v16_dev), vec);
     return launch_pdl(ctx, rope_prefill_kernel<false>, grid, dim3(256), qkv_dev, (int)tokens, n_q_heads, n_kv_heads, head_dim, cos_dev, sin_dev, pos0,
-                      k_cache_dev, v_cache_dev, static_cast<uint16_t *>(q16_dev), static_cast<uint16_t *>(k16_dev), static_cast<uint16_t *>(v16_dev));
+                      k_cache_dev, v_cache_dev, static_cast<uint16_t *>(q16_dev), static_cast<uint16_t *>(k16_dev), static_cast<uint16_t *>(v16_dev), vec);
 }
 
 cq_status cq_cast_f32_to_16(cq_ctx *ctx, const float *src_dev, int64_t count, int is_bf16, void *dst16_dev) {
@@ -1174,9 +1254,9 @@ cq_status cq_silu_mul_pairs(cq_ctx *ctx, const float *gate_up_dev, int64_t rows,
     CQ_ENTER(ctx);
     if (!gate_up_dev || !out_dev || rows < 1 || n < 1 || n > 0x7FFFFFFF || ld_out < n || (reinterpret_cast<uintptr_t>(gate_up_dev) & 7))
         return cq_fail(ctx, CQ_ERR_INVALID_ARG, "cq_silu_mul_pairs: bad arguments");
-    const int64_t total = rows * n;
-    const unsigned grid = (unsigned)((total + 255) / 256 < (int64_t)ctx->sm_count * 8 ? (total + 255) / 256 : (int64_t)ctx->sm_count * 8);
-    return launch_pdl(ctx, silu_mul_pairs_kernel, dim3(grid), dim3(256), gate_up_dev, (int)n, total, out_dev, ld_out);
+    const int vec = n % 2 == 0 && ld_out % 2 == 0 && (reinterpret_cast<uintptr_t>(gate_up_dev) & 15) == 0 && (reinterpret_cast<uintptr_t>(out_dev) & 7) == 0;
+    const unsigned gx = (unsigned)((n / (vec ? 2 : 1) + 255) / 256);
+    return launch_pdl(ctx, silu_mul_pairs_kernel, dim3(gx, (unsigned)(rows < 65535 ? rows : 65535)), dim3(256), gate_up_dev, (int)n, rows, vec, out_dev, ld_out);
 }
 
 cq_status cq_argmax(cq_ctx *ctx, const float *x_dev, int64_t rows, int64_t cols, uint32_t *out_dev) {

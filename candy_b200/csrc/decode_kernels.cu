@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(1024) rmsnorm_kernel(float *__restrict__ x, co
     float *xr = x + (int64_t)blockIdx.x * cols;
     const float *dr = ADD ? delta + (int64_t)blockIdx.x * cols : nullptr;
     float *yr = y + (int64_t)blockIdx.x * cols;
-    constexpr int HELD = 8;  // values a thread keeps: all loads of a row in flight at once, and none read twice (rows of 4096 x 128 6.9 -> us)
+    constexpr int HELD = 8;  // values a thread keeps: all loads of a row in flight at once, and none read twice (128 rows of 4096: 6.8 -> 5.4 us)
     const bool held = cols <= HELD * (int)blockDim.x;
     float v[HELD], d[HELD], w[HELD], ss = 0.0f;
     if (held) {

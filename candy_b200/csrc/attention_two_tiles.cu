@@ -395,6 +395,7 @@ __global__ void __launch_bounds__(F2_THREADS, 1)
                 *own = l;
                 meet();
                 l += *other;
+                meet();  // the next item's maxima go to the same words, and its scores do not wait for the partner's read
             }
             if (half == 0 && p.lse && row < p.seqlen_q)  // kernels/softmax.h:206: max * scale + log(sum); +inf for a row with nothing to attend to
                 p.lse[((int64_t)batch * p.h + head) * p.seqlen_q + row] = (l == 0.0f || l != l) ? INFINITY : m * p.scale + logf(l);

@@ -32,6 +32,16 @@ def test_edges(two_tiles, b, h, hk, sq, sk, d, causal, bf16):
     assert lse_err <= 2e-3, lse_err
 
 
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("d", [64, 128])
+def test_several_items_per_cta(two_tiles, d, causal):
+    """Two to three items for each CTA (2 x 64 heads x three pairs of query tiles on at most 148): the words through which the
+    halves of a row exchange maxima and sums pass from item to item."""
+    for _ in range(3):
+        err, lse_err = run_case(two_tiles, 2, 64, 8, 600, 300, d, causal, True)
+        assert err <= 1.5e-2 and lse_err <= 2e-3, (err, lse_err)
+
+
 def test_packed_strides(two_tiles):
     err, lse_err = run_case(two_tiles, 2, 4, 2, 384, 384, 128, True, False, packed=True)
     assert err <= 2e-3 and lse_err <= 2e-3

@@ -63,12 +63,15 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 
 // 2^x of two numbers on the f32 pipes: x = whole + f with |f| <= 1/2 by adding and taking off 1.5 * 2^23, 2^f by a polynomial
 // (Remez exchange for the relative error on [-1/2, 1/2]: 7.5e-8, in f32 arithmetic 2.1e-7, as ex2.approx), the whole number
-// as the exponent of a factor.  Below -127 the factor is 0; NaN stays NaN.  For x < 128.
+// as the exponent of a factor.  Below -127 the factor is 0; above 127 it stays 2^127 (a larger one would not fit the exponent),
+// which the caller's check of its sum notices as it does an infinity; NaN stays NaN.
 __device__ __forceinline__ uint64_t ex2_poly2(uint64_t x) {
     float a, b;
     unpack2(x, a, b);
     asm("max.NaN.f32 %0, %0, %1;" : "+f"(a) : "f"(-127.0f));
     asm("max.NaN.f32 %0, %0, %1;" : "+f"(b) : "f"(-127.0f));
+    asm("min.NaN.f32 %0, %0, %1;" : "+f"(a) : "f"(127.0f));
+    asm("min.NaN.f32 %0, %0, %1;" : "+f"(b) : "f"(127.0f));
     x = pack2(a, b);
     const uint64_t t = add2(x, dup2(12582912.0f)), f = fma2(add2(t, dup2(-12582912.0f)), dup2(-1.0f), x);
     uint64_t y = fma2(f, dup2(0x1.5c08e6p-10f), dup2(0x1.3d0c52p-7f));

@@ -79,6 +79,25 @@ def test_scores_that_grow_from_tile_to_tile(device, growth, causal, bf16):
     assert np.abs(lse[fin] - want_lse[fin]).max() <= 2e-3 + 2.0 ** -22 * np.abs(want_lse[fin]).max() and np.isinf(lse[~fin]).all()
 
 
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("raised", [60, 80, 95, 150, 200, 300, 400])
+def test_one_key_far_above_the_first_tile(device, raised, causal, bf16):
+    """In head h the key at column h of a half key tile, in a later tile, lies `raised` above everything before it: from there on
+    a row's softmax is that key (times 1 / (1 + about 500 e^-raised)), whichever unit evaluates its column."""
+    rng = np.random.default_rng(raised)
+    sq, sk, h, d = 260, 640, 64, 64
+    q, k, v = (rng.standard_normal((1, s, h, d)).astype(np.float32) for s in (sq, sk, sk))
+    q[..., 0], k[..., 0] = 8.0, 0.0
+    for i in range(h):
+        k[0, 128 * (2 + i % 3) + 64 * (i & 1) + i, i, 0] = raised
+    q, k, v = (from16(to16(a, bf16), bf16) for a in (q, k, v))
+    want, want_lse = an.mha_forward(q, k, v, 1.0 / np.sqrt(d), causal)
+    got, lse = attend(device, q, k, v, 1.0 / np.sqrt(d), causal, bf16, 2)
+    assert np.abs(got - want).max() <= (1.5e-2 if bf16 else 2e-3) * np.abs(want).max()
+    assert np.abs(lse - want_lse).max() <= 2e-3 + 2.0 ** -22 * np.abs(want_lse).max()
+
+
 @pytest.mark.parametrize("scale", [0.09, 0.0, -0.09])
 def test_not_finite_as_with_one_tile(device, scale):
     """Infinities and NaNs in q, k or v, and scales that are not positive (which keep one tile per CTA)."""

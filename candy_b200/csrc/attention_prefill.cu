@@ -513,26 +513,35 @@ cq_status run_fa(cq_ctx *ctx, const CUtensorMap &tq, const CUtensorMap &tk, cons
     return CQ_OK;
 }
 
-// Whether two query tiles per CTA are quicker: a step of theirs (one key tile, both query tiles) takes 4/3 of what a key tile takes
-// here (4096 keys, one item per SM: 54 and 42 us), but there are half as many items to fill the SMs with.  Counted is the busiest
-// SM's work: items are dealt out heavy first in rounds, so a full round gives each SM about its middle item, the last one its
-// first.  (us, one / two tiles: 32 heads x 1024 x 1024 causal 17.9 / 19.4, 40 heads x 900 23.5 / 19.3, 16 heads x 2048 26.3 / 32.3,
-// 32 heads x 2048 47.5 / 36.3; without a mask 32 heads x 1024 27.1 / 20.7, 8 heads x 2048 25.2 / 32.3.)
+// Whether two query tiles per CTA are quicker.  A step of theirs (one key tile, both query tiles) takes 1.5 times what a key tile takes
+// here (4096 keys, one item per SM: 62 and 44 us), but there are half as many items to fill the SMs with.  Counted is the work of
+// the busiest of five CTAs spread over the grid, as the kernels deal items out (heavy first, alternating directions), in key tiles
+// and one more per item for its start; 7/5 divides best what was measured, within 3 % of the better one over 75 shapes of 129 to 4096
+// queries but for 64 heads x 315 (11.4 / 10.3).  (us, one / two tiles: 32 heads x 1024 x 1024 causal 17.1 / 20.9, 40 heads x
+// 900 23.1 / 20.1, 32 x 1104 19.6 / 21.1, 16 x 2048 25.2 / 35.0, 32 x 2048 47.4 / 39.2; without a mask 32 heads x 1024 26.3 / 21.0,
+// 8 x 2048 24.0 / 34.6.)
 bool two_tiles_win(const FaParams &p, int sms) {
-    const int64_t hb = (int64_t)p.h * p.b;
     if (p.seqlen_q <= FA_M) return false;
-    auto busiest = [&](int64_t rows) {  // key tiles, with `rows` query rows per item
-        const int64_t nq = (p.seqlen_q + rows - 1) / rows, items = nq * hb, all = (p.seqlen_k + FA_N - 1) / FA_N;
-        int64_t sum = 0;
-        for (int64_t first = 0; first < items; first += sms) {
-            const int64_t at = first + sms <= items ? first + sms / 2 : first, last = std::min<int64_t>((nq - at / hb) * rows, p.seqlen_q);  // rows before this
-            const int64_t lim = p.causal ? last + p.seqlen_k - p.seqlen_q : p.seqlen_k;  // keys that the item's last row sees
-            sum += std::max<int64_t>(0, std::min(all, (lim + FA_N - 1) / FA_N));
-        }
-        return sum;
-    };
+    const int64_t hb = (int64_t)p.h * p.b;
     if ((p.seqlen_q + 2 * FA_M - 1) / (2 * FA_M) * hb >= 16 * (int64_t)sms) return true;  // both fill the SMs
-    return 4 * busiest(2 * FA_M) < 3 * busiest(FA_M);
+    const int all = (p.seqlen_k + FA_N - 1) / FA_N, off = p.seqlen_k - p.seqlen_q, rows_up = (p.seqlen_q + FA_M - 1) / FA_M * FA_M;
+    auto busiest = [&](int rows) {  // with `rows` query rows per item
+        const int nq = (p.seqlen_q + rows - 1) / rows, heads = (int)hb, items = nq * heads, grid = std::min(items, sms);
+        int most = 0;
+        for (int i = 0; i < 5; ++i) {
+            const int cta = i * (grid - 1) / 4;
+            int sum = 0;
+            for (int rd = 0; rd * grid < items; ++rd) {
+                const int w = (rd & 1) ? (rd + 1) * grid - 1 - cta : rd * grid + cta;
+                if (w >= items) continue;
+                const int lim = p.causal ? std::min((nq - w / heads) * rows, rows_up) + off : p.seqlen_k;  // keys that the item's last row sees
+                sum += 1 + std::max(0, std::min(all, (lim + FA_N - 1) / FA_N));
+            }
+            most = std::max(most, sum);
+        }
+        return most;
+    };
+    return 7 * busiest(2 * FA_M) < 5 * busiest(FA_M);
 }
 
 }  // namespace
@@ -603,7 +612,7 @@ cq_status cq_flash_attention(cq_ctx *ctx, void *q_ptr, void *k_ptr, void *v_ptr,
     // persistent CTAs, one per SM (the kernel's shared memory allows no more), each walking its share of the work items
     const int64_t items = (int64_t)((seqlen_q + FA_M - 1) / FA_M) * h * b;
     const dim3 grid((unsigned)(items < ctx->sm_count ? items : ctx->sm_count));
-    if (v_direct && ctx->tune.fa_two_tiles && softmax_scale > 0.0f && seqlen_k <= (bf ? 65536u : 16384u) &&
+    if (v_direct && ctx->tune.fa_two_tiles && softmax_scale > 0.0f && seqlen_k <= (bf ? 8192u : 2048u) &&
         (ctx->tune.fa_two_tiles == 2 || two_tiles_win(p, ctx->sm_count)))
         return launch_fmha_two_tiles(ctx, tq, tk, tv, p, (int)d, bf);
     if (v_direct) {

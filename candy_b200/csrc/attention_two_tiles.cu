@@ -1,5 +1,5 @@
 // Prefill attention with two tiles of 128 query rows per CTA, the same contract as attention_prefill.cu (which serves small
-// problems, V tiles that the tensor maps cannot address, and very long rows of keys).
+// problems, V tiles that the tensor maps cannot address, and long rows of keys).
 //
 // One tile alone leaves the tensor core idle during its softmax and the other way round.  Here two tiles of the same head take
 // turns, and each K and V tile is fetched once for both:
@@ -8,20 +8,19 @@
 //               thread execute in order); the whole warp runs the loop and one lane issues
 //   warps 4-11  softmax of tile 0, warps 12-19 of tile 1: thread = (query row, half of the scores of a key tile).  p = ex2 of
 //               the scaled difference goes back as 16-bit pairs over the first half of the scores' own tensor-memory columns
-// The output accumulates in tensor memory over all key tiles.  p is taken relative to a reference m of the row, its maximum in
-// the first key tile, and no tile's maximum is looked for after that as long as the tile's sums of p stay below 2^13, which
-// bounds every p.  Where one does not, the rows get new references and their accumulators are rescaled (by the softmax threads,
-// between the products of two key tiles).  f32, f16 and bf16 hold such p with the relative precision that they have below 1;
-// the row's largest p is no longer exactly 1, which leaves 2 % more rounding of p in the result (2.05e-3 -> 2.09e-3 of it in bf16,
-// 2.55e-4 -> 2.60e-4 in f16, against f64).
-// The tensor core truncates when it adds, 4.6e-9 of the sum per key for values of one sign: 1.9e-5 at 4096 keys.  The caller
-// keeps rows beyond 16384 (f16) / 65536 (bf16) keys away, where that would be seen beside the rounding of p.
+// p is taken relative to the row's maximum so far, the row's largest p is exactly 1, and the accumulators are rescaled wherever a
+// key tile raises a maximum, by the softmax threads before they hand their p over: an output as near to 64 bits as one tile's.
+// (With a reference that moves only when p would pass 2^13 the scores' maxima and the rescaling are saved, 453 us for 517 in the
+// first shape below, but the largest p is rounded too: 2.05e-3 -> 2.09e-3 of the result in bf16, 2.56e-4 -> 2.61e-4 in f16.)
+// The output accumulates in tensor memory over all key tiles, where the tensor core truncates as it adds: 6e-9 of the sum per key
+// for values of one sign, 1e-9 for mixed ones.  Rows of up to 2048 keys (f16) / 8192 (bf16) come here, where that adds at most
+// 0.3 % to the error that the rounding of p and of the result leaves (positive values, f16, 4096 keys: 1.767e-4 -> 1.784e-4, four
+// times as much as at 2048; mixed ones 2.855e-4 either way).
 //
-// 2 x 64/8 heads x 4096 causal bf16, one tile per CTA 600 us -> 453; 32 heads x 2048 causal f16 47.5 -> 36.  The tensor pipe is
-// 62 % active, at 1.7 GHz (the power limit).  What was tried (us, first shape): one thread per row 472; the control warps behind
-// the softmax warps 466; every p on the special-function unit 481, a third or a fifth on the f32 pipes 453 / 457; P handed over
-// in halves and the maximum of every tile 500; an issuing warp per tile 523, the two in strict turns 493 (a faster issue brings
-// the tiles into step, and both softmaxes then run while the tensor core has nothing to do).
+// us, one tile per CTA -> two, sustained (in bursts): 2 x 64/8 heads x 4096 causal bf16 645 -> 557 (616 -> 517); 32 heads x 2048 causal
+// f16 47 -> 39; 32/8 heads x 4096 of 64 causal bf16 141 -> 103.  What was tried (us, first shape, bursts): every p on the
+// special-function unit 516, a half / a third / a quarter / a fifth on the f32 pipes 550 / 517 / 518 / 522 (32 x 2048: 46.5, 48, 45,
+// 45.5, 46).
 // Persistent CTAs, items (256 query rows, head, batch) heavy first and in alternating directions, as in attention_prefill.cu:
 // rings, phases and tensor memory carry on from item to item.  Every wait is bounded; tensor memory is always freed.
 #include "attention.cuh"
@@ -63,15 +62,12 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 
 // 2^x of two numbers on the f32 pipes: x = whole + f with |f| <= 1/2 by adding and taking off 1.5 * 2^23, 2^f by a polynomial
 // (Remez exchange for the relative error on [-1/2, 1/2]: 7.5e-8, in f32 arithmetic 2.1e-7, as ex2.approx), the whole number
-// as the exponent of a factor.  Below -127 the factor is 0; above 127 it stays 2^127 (a larger one would not fit the exponent),
-// which the caller's check of its sum notices as it does an infinity; NaN stays NaN.
+// as the exponent of a factor.  Below -127 the factor is 0; NaN stays NaN.  For x < 128: here no x is above a rounding of 0.
 __device__ __forceinline__ uint64_t ex2_poly2(uint64_t x) {
     float a, b;
     unpack2(x, a, b);
     asm("max.NaN.f32 %0, %0, %1;" : "+f"(a) : "f"(-127.0f));
     asm("max.NaN.f32 %0, %0, %1;" : "+f"(b) : "f"(-127.0f));
-    asm("min.NaN.f32 %0, %0, %1;" : "+f"(a) : "f"(127.0f));
-    asm("min.NaN.f32 %0, %0, %1;" : "+f"(b) : "f"(127.0f));
     x = pack2(a, b);
     const uint64_t t = add2(x, dup2(12582912.0f)), f = fma2(add2(t, dup2(-12582912.0f)), dup2(-1.0f), x);
     uint64_t y = fma2(f, dup2(0x1.5c08e6p-10f), dup2(0x1.3d0c52p-7f));
@@ -304,87 +300,76 @@ __global__ void __launch_bounds__(F2_THREADS, 1)
             item_at(w, q0, head, batch, nt);
             const int n = nt[x], row = q0 + x * FA_M + r;              // global query index
             const int causal_lim = p.causal ? row + off : 0x7FFFFFFF;  // last visible key
-            float m = 0.0f;                                            // the row's reference (raw scores)
+            float m = -INFINITY;                                       // the row's maximum so far (raw scores)
             float l = 0.0f;                                            // sum of this half
             for (int t = 0; t < n; ++t, ++g) {
                 wait(&s_full[x], g);
                 const int kmax = min(p.seqlen_k - 1, causal_lim) - t * FA_N - half * HC;  // columns > kmax of this half are masked
                 const bool cut = !__all_sync(0xffffffffu, kmax >= HC - 1);
-                uint32_t pk[HC / 2];
-                float l_tile;
-                for (bool refer = t == 0;;) {
-                    uint32_t sv[HC];
+                uint32_t sv[HC];
 #pragma unroll
-                    for (int c = 0; c < HC / 32; ++c) tmem_ld32_async(s_addr + c * 32, sv + c * 32);
-                    tmem_wait_ld();
-                    if (cut)
+                for (int c = 0; c < HC / 32; ++c) tmem_ld32_async(s_addr + c * 32, sv + c * 32);
+                tmem_wait_ld();
+                if (cut)
 #pragma unroll
-                        for (int i = 0; i < HC; ++i) sv[i] = i <= kmax ? sv[i] : 0xFF800000u;
-                    if (refer) {
-                        float m4[4];  // independent chains
+                    for (int i = 0; i < HC; ++i) sv[i] = i <= kmax ? sv[i] : 0xFF800000u;
+                // the row's maximum so far (the partner's half through shared memory: it has read this word's last value before
+                // its part of the last P was handed over, and these scores were computed after that)
+                float m4[4];  // independent chains
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) m4[u] = __uint_as_float(sv[u]);
+                for (int u = 0; u < 4; ++u) m4[u] = __uint_as_float(sv[u]);
 #pragma unroll
-                        for (int i = 4; i + 8 <= HC; i += 8) {
+                for (int i = 4; i + 8 <= HC; i += 8) {
 #pragma unroll
-                            for (int u = 0; u < 4; ++u) m4[u] = max3(m4[u], __uint_as_float(sv[i + u]), __uint_as_float(sv[i + 4 + u]));
-                        }
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) m4[u] = fmaxf(m4[u], __uint_as_float(sv[HC - 4 + u]));
-                        *own = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
-                        meet();
-                        const float m_tile = fmaxf(*own, *other);
-                        if (t == 0) {
-                            m = m_tile == -INFINITY ? 0.0f : m_tile;  // (nothing visible, or scores of -inf: p is 0 for any reference)
-                        } else {
-                            const float m_new = fmaxf(m, m_tile), alpha = fast_ex2((m - m_new) * p.scale_log2);
-                            m = m_new;
-                            l *= alpha;
-#pragma unroll 1
-                            for (int c = 0; c < HD / 16; ++c) {
-                                uint32_t o[16];
-                                tmem_ld16(o_addr + c * 16, o);
-#pragma unroll
-                                for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                                tmem_st16(o_addr + c * 16, o);
-                            }
-                            tmem_wait_st();
-                        }
-                    }
-                    // p = exp2(s * scale_log2 - m * scale_log2), summed in f32, as 16-bit pairs.  Every third pair takes the f32
-                    // pipes, which have less to do than the special-function unit with its 16 lanes a cycle and SM.
-                    const uint64_t c2 = dup2(p.scale_log2), mb2 = dup2(-m * p.scale_log2);
-                    uint64_t sum[2] = {0, 0};
-#pragma unroll
-                    for (int i = 0; i < HC / 2; ++i) {
-                        const uint64_t x2 = fma2(pack2(__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])), c2, mb2);
-                        float e0, e1;
-                        if (i % 3 == 2) {
-                            unpack2(ex2_poly2(x2), e0, e1);
-                        } else {
-                            unpack2(x2, e0, e1);
-                            e0 = fast_ex2(e0), e1 = fast_ex2(e1);
-                        }
-                        sum[i & 1] = add2(sum[i & 1], pack2(e0, e1));
-                        pk[i] = pack16<BF16>(e0, e1);
-                    }
-                    float a, b;
-                    unpack2(add2(sum[0], sum[1]), a, b);
-                    l_tile = a + b;
-                    // A sum below 2^13 has no term above it.  Otherwise the 32 rows get new references and their products so far
-                    // are rescaled, once they are complete; the scores are still there, p has not left the registers.  (The
-                    // barrier is needed anyway: p goes where the other half's scores were.)
-                    int again;
-                    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbarrier.cta.red.or.pred q, %2, 64, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
-                                 : "=r"(again)
-                                 : "r"((int)!(l_tile < 8192.0f)), "r"(pair)
-                                 : "memory");
-                    if (refer || !again) break;
-                    refer = true;
-                    wait(&o_done[x], g - 1);
+                    for (int u = 0; u < 4; ++u) m4[u] = max3(m4[u], __uint_as_float(sv[i + u]), __uint_as_float(sv[i + 4 + u]));
                 }
-                l += l_tile;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) m4[u] = fmaxf(m4[u], __uint_as_float(sv[HC - 4 + u]));
+                const float m_half = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+                *own = m_half;
+                meet();  // (needed for P as well, which goes where the other half's scores were)
+                const float m_new = max3(m, m_half, *other), m_use = m_new == -INFINITY ? 0.0f : m_new;  // (nothing to see yet: every p is 0)
+                const float alpha = fast_ex2((m - m_use) * p.scale_log2);  // m = -inf gives 0
+                m = m_new;
+                // p = exp2(s * scale_log2 - m * scale_log2), summed in f32, as 16-bit pairs.  Every third pair takes the f32
+                // pipes, which have less to do than the special-function unit with its 16 lanes a cycle and SM.
+                const uint64_t c2 = dup2(p.scale_log2), mb2 = dup2(-m_use * p.scale_log2);
+                uint64_t sum[2] = {0, 0};
+                uint32_t pk[HC / 2];
+#pragma unroll
+                for (int i = 0; i < HC / 2; ++i) {
+                    const uint64_t x2 = fma2(pack2(__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])), c2, mb2);
+                    float e0, e1;
+                    if (i % 3 == 2) {
+                        unpack2(ex2_poly2(x2), e0, e1);
+                    } else {
+                        unpack2(x2, e0, e1);
+                        e0 = fast_ex2(e0), e1 = fast_ex2(e1);
+                    }
+                    sum[i & 1] = add2(sum[i & 1], pack2(e0, e1));
+                    pk[i] = pack16<BF16>(e0, e1);
+                }
                 tmem_st32(p_addr, pk);
+                float a, b;
+                unpack2(add2(sum[0], sum[1]), a, b);
+                l = fmaf(l, alpha, a + b);
+                // The products so far are complete: the scores above were issued behind them.
+                if (t > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) {
+                    const uint64_t alpha2 = dup2(alpha);
+#pragma unroll
+                    for (int c = 0; c < HD / 32; ++c) {
+                        uint32_t o[32];
+                        tmem_ld32_async(o_addr + c * 32, o);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            float lo, hi;
+                            unpack2(mul2(pack2(__uint_as_float(o[2 * i]), __uint_as_float(o[2 * i + 1])), alpha2), lo, hi);
+                            o[2 * i] = __float_as_uint(lo), o[2 * i + 1] = __float_as_uint(hi);
+                        }
+                        tmem_st32(o_addr + c * 32, o);
+                    }
+                }
                 tmem_wait_st();
                 tc_fence_before();
                 __syncwarp();
@@ -395,6 +380,7 @@ __global__ void __launch_bounds__(F2_THREADS, 1)
                 waited_prior = true;
             }
             if (n > 0) {
+                meet();  // the partner has read the last maximum
                 *own = l;
                 meet();
                 l += *other;

@@ -50,10 +50,10 @@ struct GbCfg {
     static constexpr int kBlockBytes = QT == CQ_Q4_0 ? kQ4Bytes : kQ8Bytes;
     static constexpr int kRowChunk = 8 * kBlockBytes;          // 144 / 272 bytes
     static constexpr int kWBytes = GP_ROWS * kRowChunk;
-    static constexpr int kWStages = QT == CQ_Q4_0 ? (kFix ? 3 : 4) : 2;
+    static constexpr int kWStages = QT == CQ_Q4_0 ? 3 : 2;
     static constexpr int kBoxBytes = NB * 128;                 // 64 k of the batch rows
     static constexpr int kXBytes = 2 * kBoxBytes;              // hi, lo
-    static constexpr int kXStages = 4;
+    static constexpr int kXStages = 4;                         // a chunk's units: its first one, with the corrections, is always in stage 0
     static constexpr int kFixBytes = kFix ? NB * 64 : 0;       // a chunk's corrections, two buffers
     static constexpr int kOnesBytes = kFix ? GP_ROWS * 128 : 0;
     static constexpr int kScaleBytes = GB_SCALES * GP_ROWS * 4;
@@ -244,7 +244,9 @@ __global__ void __launch_bounds__(GbCfg<QT, NB>::kThreads, 1)
         }
         for (int s = 0; s < XST; ++s) {
             mbar_init(smem_u32(&x_full[s]), 1);
-            mbar_init(smem_u32(&u_done[s]), BPS == 1 ? 2 : 1);  // the unit's MMAs have read its slab and its A buffer
+            // the unit's MMAs have read its slab and its A buffer (and where the corrections come with a unit that one of the two
+            // issuing warps has no part in, that warp has seen it come: the barrier is never two phases ahead of a wait)
+            mbar_init(smem_u32(&u_done[s]), BPS == 1 || (Cfg::kFix && s == 0) ? 2 : 1);
         }
         for (int b = 0; b < GB_A; ++b) mbar_init(smem_u32(&a_full[b]), 4);
         for (int s = 0; s < GB_SLOTS; ++s) {
@@ -349,6 +351,7 @@ __global__ void __launch_bounds__(GbCfg<QT, NB>::kThreads, 1)
                             ok = false;
                             break;
                         }
+                        if (BPS == 2 && !mine && lane == 0) mbar_arrive(smem_u32(&u_done[s]));
                     }
                     if (mine) {
                         tc_fence_after();

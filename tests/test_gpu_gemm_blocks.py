@@ -38,7 +38,8 @@ def terms(qt, order, x, blocks, n):
 
 
 @pytest.mark.parametrize("qt,order", QT_ORDERS)
-@pytest.mark.parametrize("m,n,k", [(33, 1, 256), (64, 127, 512), (65, 128, 768), (128, 129, 256), (129, 700, 2304), (300, 2000, 512), (70, 9000, 1024)])
+@pytest.mark.parametrize("m,n,k", [(33, 1, 256), (64, 127, 512), (65, 128, 768), (128, 129, 256), (129, 700, 2304), (300, 2000, 512), (70, 9000, 1024),
+                                   (40, 300, 8192)])
 def test_edges(device, qt, order, m, n, k):
     rng = np.random.default_rng(m + n + k + order)
     blocks = oc.quantize(qt, order, (rng.standard_normal((n, k)) * 0.02).astype(np.float32))

@@ -4,11 +4,13 @@
 //
 // q: the block's whole numbers, exact in f16.  hi + lo: the numbers d8 * q8 that quantize_q8_1 makes of an activation row
 // (quantized.cu:3521-3558), 19 bits; scaled by a power of two so that the row's largest value sits just below 2^15 the sum of
-// two f16 numbers holds them exactly.  Each block's dots are a product of their own in a rotating slot of tensor memory, two
-// K = 16 steps with lo and two with hi (lo first: the tensor core truncates when it adds, and so it does on the small numbers);
-// the epilogue multiplies by d and adds up in f32 registers, one fused multiply-add per result.  Against Q4_0 a block's dot is
-// sumi d8 - 8 s8 with the block's sum s8 in f16 (vec_dot_q4_0_q8_1, :1919-1941), which differs from sum (q - 8) d8 q8 by
-// c = 8 (sum d8 q8 - s8): a fifth K = 16 step multiplies (c_hi, c_lo) / 512 by 512.
+// two f16 numbers holds them exactly, whatever a block's size beside its row's: d8 is an f16 number, so the values are multiples
+// of 2^-24 before that scaling, and lo is kept times 2^11.  Each block's dots are a product of their own in a rotating slot of
+// tensor memory, two K = 16 steps with lo, then two with hi, the first of which takes the accumulator times 2^-11 (lo first: the
+// tensor core truncates when it adds, and so it does on the small numbers); the epilogue multiplies by d and adds up in f32
+// registers, one fused multiply-add per result.  Against Q4_0 a block's dot is sumi d8 - 8 s8 with the block's sum s8 in f16
+// (vec_dot_q4_0_q8_1, :1919-1941), which differs from sum (q - 8) d8 q8 by c = 8 (sum d8 q8 - s8): a fifth K = 16 step between
+// the two multiplies (c_hi, c_lo 2^11) / 512 by (512, 1/4).
 //
 // The int8 GEMM (gemm_i8_tmem.cu), which served these batches and still serves the small ones, has exact whole-number dots but
 // scales them by both operands' block scales in the epilogue, and an activation scale, the same in every lane, costs a warp
@@ -31,8 +33,9 @@
 // Work is the list of (tile, 256-wide chunk of k), cut into equal contiguous shares per CTA; partial tiles go to scratch and
 // a small kernel adds them in order (the same bits from run to run).  Every wait is bounded.
 //
-// Left to the epilogue, which computes them from the blocks with whole-number dots: weight rows with an infinite or NaN scale,
-// and activation rows that 19 bits below their largest value do not hold (the pre-pass hands over a negative scale).
+// Left to the epilogue warps, behind all other work of the CTA, when nobody waits for them: weight rows with an infinite or NaN scale,
+// and activation rows with a d8 or s8 that f16 does not hold (values beyond 8.3e6, blocks that sum up to 65520; the pre-pass hands
+// over a negative scale).  None of their results is finite, and the blocks concerned alone say which infinity or NaN each is.
 #include <type_traits>
 
 #include "gemm_raw.cuh"
@@ -43,6 +46,9 @@ constexpr int GB_SLOTS = 3;    // of 128 tensor-memory columns
 constexpr int GB_EPW = 8;      // epilogue warps
 constexpr int GB_SCALES = 8;   // units in the ring of weight scales (see the kernel)
 constexpr int GB_A = 4;        // A buffers of 32 tensor-memory columns (a unit)
+constexpr int GB_LO_BITS = 11; // lo is kept times 2^11
+constexpr float GB_LO = 1 << GB_LO_BITS;
+constexpr int GB_LIST = 8192;  // blocks of a row looked over at a time for what is not finite
 
 template <int QT, int NB>
 struct GbCfg {
@@ -63,16 +69,17 @@ struct GbCfg {
     static constexpr size_t kSmem = (size_t)kXStages * kXBytes + 2 * kFixBytes + kOnesBytes + (size_t)kWStages * kWBytes + kScaleBytes + 1024 + 8 * kBars + 16;
     static constexpr int kACol0 = 128 * GB_SLOTS;
     static_assert(kSmem <= 232448 && kACol0 + 32 * GB_A <= 512, "shared / tensor memory");
+    static_assert(kXStages * kXBytes >= 4 * (GB_LIST + 129), "room for a list of blocks");
 };
 
 // What quantize_q8_1 makes of a value (true division, ties away from zero).
 __device__ __forceinline__ float gb_q8(float v, float d) { return (float)(int)roundf(__fdiv_rn(v, d)); }
 
-// One CTA per row: largest magnitude, then d8 q8 2^e = hi + lo with 2^14 <= amax 2^e < 2^15 (e = 0 for a row of zeros).
-// lo ends at f16's last bit, 2^-24: the 19 bits are all there in 32-blocks whose largest value reaches 2^-6.  A row with a
-// smaller one (2^20 below the row's largest), or with a d8 or s8 that is not finite, gets a negative scale, and the epilogue
-// computes it with whole-number dots.
-// fix: [m][k / 8], per 128 k the four blocks' (c_hi, c_lo) and eight zeros.
+// One CTA per row: largest magnitude, then d8 q8 2^e = hi + lo 2^-11 with 2^14 <= amax 2^e < 2^15 (e = 0 for a row of zeros).
+// Exact: d8 q8 has 18 bits and is a multiple of 2^-24, and where d8 is finite (amax < 2^23) e is at least -8, so lo 2^11 is a
+// multiple of 2^-21; a d8 below f16's normal numbers is up to twice amax / 127 and leaves hi below 65024 and lo 2^11 below 2^15.
+// A row with a d8 or s8 that is not finite gets a negative scale, which leaves it to the epilogue warps.
+// fix: [m][k / 8], per 128 k the four blocks' (c_hi, c_lo 2^11) and eight zeros.
 __global__ void __launch_bounds__(256) gb_x_q8_kernel(const float *__restrict__ x, int64_t k, int64_t ldx, int order, __half *__restrict__ hi,
                                                        __half *__restrict__ lo, __half *__restrict__ fix, float *__restrict__ scale) {
     pdl_launch_dependents();
@@ -100,7 +107,7 @@ __global__ void __launch_bounds__(256) gb_x_q8_kernel(const float *__restrict__ 
     int e = 0;
     if (amax > 0.0f && amax < INFINITY) e = min(14 - ilogbf(amax), 126);
     const float up = __int_as_float((127 + e) << 23);  // e in [-113, 126]
-    bool low = false, odd = false;
+    bool odd = false;
 #pragma unroll 4
     for (int64_t o8 = threadIdx.x; o8 < k / 8; o8 += 256) {
         float v[8];
@@ -109,7 +116,6 @@ __global__ void __launch_bounds__(256) gb_x_q8_kernel(const float *__restrict__ 
         float top = fmaxf(fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))), fmaxf(fmaxf(fabsf(v[4]), fabsf(v[5])), fmaxf(fabsf(v[6]), fabsf(v[7]))));
         top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
         top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
-        low |= top > 0.0f && top * up < 0x1p-6f;
         const float d = __fdiv_rn(top, 127.0f), dh = __half2float(__float2half_rn(d));
         float q[8];
 #pragma unroll
@@ -140,12 +146,12 @@ __global__ void __launch_bounds__(256) gb_x_q8_kernel(const float *__restrict__ 
             qs += __shfl_xor_sync(0xffffffffu, qs, 1);
             qs += __shfl_xor_sync(0xffffffffu, qs, 2);
             const float sh = __half2float(__float2half_rn(s)), c = __fsub_rn(8.0f * (dh * qs), 8.0f * sh) * up * 0x1p-9f;
-            odd |= fabsf(c) > 65000.0f;  // (with a d8 below f16's normal numbers c reaches 768 amax; an infinite s8)
+            odd |= !(fabsf(c) < 65000.0f);  // an infinite s8, or a NaN one (with a d8 below f16's normal numbers c reaches 768 amax 2^e / 512, 49152)
             const int64_t blk = o8 >> 2;
             __half *dst = fix + row * (k / 8) + (blk >> 2) * 16;
             if ((o8 & 3) == 0) {
                 const __half ch = __float2half_rn(c);
-                *reinterpret_cast<__half2 *>(dst + 2 * (blk & 3)) = __halves2half2(ch, __float2half_rn(c - __half2float(ch)));
+                *reinterpret_cast<__half2 *>(dst + 2 * (blk & 3)) = __halves2half2(ch, __float2half_rn((c - __half2float(ch)) * GB_LO));
             } else if ((o8 & 3) == 1) {
                 *reinterpret_cast<uint32_t *>(dst + 8 + 2 * (blk & 3)) = 0;
             }
@@ -158,48 +164,110 @@ __global__ void __launch_bounds__(256) gb_x_q8_kernel(const float *__restrict__ 
         for (int j = 0; j < 4; ++j) {
             const float a = v[2 * j] * up, b = v[2 * j + 1] * up;
             const __half2 h = __floats2half2_rn(a, b);
-            const __half2 l = __floats2half2_rn(a - __low2float(h), b - __high2float(h));
+            const __half2 l = __floats2half2_rn((a - __low2float(h)) * GB_LO, (b - __high2float(h)) * GB_LO);
             wh[j] = *reinterpret_cast<const uint32_t *>(&h);
             wl[j] = *reinterpret_cast<const uint32_t *>(&l);
         }
         *reinterpret_cast<uint4 *>(hi + row * k + o8 * 8) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
         *reinterpret_cast<uint4 *>(lo + row * k + o8 * 8) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
     }
-    low = __syncthreads_or((low && amax < INFINITY) || odd);
-    if (threadIdx.x == 0) scale[row] = (low ? -1.0f : 1.0f) * __int_as_float((127 - e) << 23);
+    odd = __syncthreads_or(odd);
+    if (threadIdx.x == 0) scale[row] = (odd ? -1.0f : 1.0f) * __int_as_float((127 - e) << 23);
 }
 
-// A dot product over blocks [b0, b1) as the reference computes it, for rows of either operand that the tensor core does not take.
-template <int QT>
-__device__ __noinline__ float gb_plain_dot(const uint8_t *wrow, const float *xrow, int order, int b0, int b1) {
-    constexpr int BB = QT == CQ_Q4_0 ? kQ4Bytes : kQ8Bytes;
-    float acc = 0.0f;
-    for (int b = b0; b < b1; ++b) {
-        const unsigned short *blk = reinterpret_cast<const unsigned short *>(wrow + (int64_t)b * BB);
-        const float d = __half2float(__ushort_as_half(blk[0])), *xb = xrow + (int64_t)b * kQK;  // x: 16-byte aligned rows
-        float s[16], top = 0.0f, d8, dot = 0.0f;
-        for (int i = 0; i < 32; ++i) top = fmaxf(top, fabsf(xb[i]));
-        d8 = __fdiv_rn(top, 127.0f);
-        for (int i = 0; i < 16; ++i) s[i] = __fadd_rn(xb[i], xb[i + 16]);
-        for (int o = 8; o > 0; o >>= 1)
-            for (int i = 0; i < o; ++i) s[i] = __fadd_rn(s[i], s[i + o]);
-        for (int j = 0; j < (BB - 2) / 2; ++j) {
-            const int two = blk[1 + j];
-            if (QT == CQ_Q4_0) {
-                for (int h = 0; h < 4; ++h) {  // byte 2j (+1): its low and its high nibble
-                    const int byte = 2 * j + (h >> 1), i = order == CQ_ORDER_GO_INTERLEAVED ? 2 * byte + (h & 1) : byte + 16 * (h & 1);
-                    dot += (float)((two >> (8 * (h >> 1) + 4 * (h & 1))) & 15) * (top == 0.0f ? 0.0f : gb_q8(xb[i], d8));
-                }
-            } else {
-                dot += (float)(signed char)(two & 0xFF) * (top == 0.0f ? 0.0f : gb_q8(xb[2 * j], d8));
-                dot += (float)(signed char)(two >> 8) * (top == 0.0f ? 0.0f : gb_q8(xb[2 * j + 1], d8));
-            }
-        }
-        d8 = __half2float(__float2half_rn(d8));
-        if (QT == CQ_Q4_0) acc = fmaf(d, fmaf(dot, d8, -8.0f * __half2float(__float2half_rn(s[0]))), acc);
-        else acc = fmaf(d * d8, dot, acc);
+// Results that are not finite.  A weight row with an infinite or NaN scale, or an activation row with such a d8 or s8, has none that
+// are, and its other blocks, whose terms are finite, have no say in which: only the terms of those blocks are added up.
+
+// d8 and s8 of a block of 32 values (16-byte aligned) as the reference computes them, before their rounding to f16.
+__device__ __forceinline__ void gb_block_scales(const float *xb, float &d8, float &s8) {
+    float s[16], top = 0.0f;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const float4 f = reinterpret_cast<const float4 *>(xb)[u], g = reinterpret_cast<const float4 *>(xb)[4 + u];
+        top = fmaxf(top, fmaxf(fmaxf(fmaxf(fabsf(f.x), fabsf(f.y)), fmaxf(fabsf(f.z), fabsf(f.w))), fmaxf(fmaxf(fabsf(g.x), fabsf(g.y)), fmaxf(fabsf(g.z), fabsf(g.w)))));
+        s[4 * u] = __fadd_rn(f.x, g.x), s[4 * u + 1] = __fadd_rn(f.y, g.y), s[4 * u + 2] = __fadd_rn(f.z, g.z), s[4 * u + 3] = __fadd_rn(f.w, g.w);
     }
-    return acc;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+        for (int u = 0; u < o; ++u) s[u] = __fadd_rn(s[u], s[u + o]);
+    d8 = __fdiv_rn(top, 127.0f), s8 = s[0];
+}
+__device__ __forceinline__ bool gb_odd_half(unsigned short h) { return (h & 0x7C00) == 0x7C00; }
+template <int QT>
+__device__ __forceinline__ bool gb_odd_block(const float *xb) {
+    float d8, s8;
+    gb_block_scales(xb, d8, s8);
+    return gb_odd_half(__half_as_ushort(__float2half_rn(d8))) || (QT == CQ_Q4_0 && gb_odd_half(__half_as_ushort(__float2half_rn(s8))));
+}
+// A block's term.
+template <int QT>
+__device__ __noinline__ float gb_term(const uint8_t *block, const float *xb, int order) {
+    constexpr int BB = QT == CQ_Q4_0 ? kQ4Bytes : kQ8Bytes;
+    const unsigned short *blk = reinterpret_cast<const unsigned short *>(block);
+    float d8, s8, dot = 0.0f;
+    gb_block_scales(xb, d8, s8);
+    auto q8 = [&](int i) { return d8 == 0.0f ? 0.0f : gb_q8(xb[i], d8); };
+    for (int j = 0; j < (BB - 2) / 2; ++j) {
+        const int two = blk[1 + j];
+        if (QT == CQ_Q4_0) {
+            for (int h = 0; h < 4; ++h) {  // byte 2j (+1): its low and its high nibble
+                const int byte = 2 * j + (h >> 1);
+                dot += (float)((two >> (8 * (h >> 1) + 4 * (h & 1))) & 15) * q8(order == CQ_ORDER_GO_INTERLEAVED ? 2 * byte + (h & 1) : byte + 16 * (h & 1));
+            }
+        } else {
+            dot += (float)(signed char)(two & 0xFF) * q8(2 * j) + (float)(signed char)(two >> 8) * q8(2 * j + 1);
+        }
+    }
+    const float d = __half2float(__ushort_as_half(blk[0])), dh = __half2float(__float2half_rn(d8));
+    return QT == CQ_Q4_0 ? d * fmaf(dot, dh, -8.0f * __half2float(__float2half_rn(s8))) : d * dh * dot;
+}
+// Weight rows j0 .. j0 + 127 (below p.n) by batch row c over blocks [b0, b1), the terms of the batch row's blocks that are not
+// finite: the 256 epilogue threads (t) together.  out[j] = (bias +) their sum.  `list`: GB_LIST + 129 words.
+template <int QT>
+__device__ __noinline__ void gb_odd_row(const GpParams &p, int j0, int c, int b0, int b1, int *list, float *out, bool bias, int t) {
+    constexpr int BB = QT == CQ_Q4_0 ? kQ4Bytes : kQ8Bytes;
+    int *count = list + GB_LIST;
+    float *sum_s = reinterpret_cast<float *>(count + 1);
+    const float *xrow = p.x + (int64_t)c * p.ldx;
+    const int r = t & 127, j = j0 + r;
+    const uint8_t *wrow = p.w + (int64_t)j * (p.k / kQK) * BB;
+    float sum = 0.0f;
+    for (int from = b0; from < b1; from += GB_LIST) {
+        const int to = min(b1, from + GB_LIST);
+        asm volatile("barrier.cta.sync 1, 256;" ::: "memory");  // the list before is done with
+        if (t == 0) *count = 0;
+        asm volatile("barrier.cta.sync 1, 256;" ::: "memory");
+        for (int b = from + t; b < to; b += 256)
+            if (gb_odd_block<QT>(xrow + (int64_t)b * kQK)) list[atomicAdd(count, 1)] = b;
+        asm volatile("barrier.cta.sync 1, 256;" ::: "memory");
+        const int n = *count;
+        if (j < p.n)
+            for (int i = t >> 7; i < n; i += 2) sum += gb_term<QT>(wrow + (int64_t)list[i] * BB, xrow + (int64_t)list[i] * kQK, p.order);
+    }
+    if (t >= 128) sum_s[r] = sum;
+    asm volatile("barrier.cta.sync 1, 256;" ::: "memory");
+    if (t < 128 && j < p.n) out[r] = (bias ? p.bias[j] : 0.0f) + (sum + sum_s[r]);
+}
+// Weight row j by batch rows c0 .. c0 + columns - 1 over blocks [b0, b1), the terms of the weight row's blocks whose scale is not
+// finite: a warp.  Added to what is there for batch rows of the kind above.
+template <int QT>
+__device__ __noinline__ void gb_odd_weights(const GpParams &p, int j, int c0, int columns, int b0, int b1, float *out, int64_t ld, bool bias, int lane) {
+    constexpr int BB = QT == CQ_Q4_0 ? kQ4Bytes : kQ8Bytes;
+    const uint8_t *wrow = p.w + (int64_t)j * (p.k / kQK) * BB;
+    for (int c = lane; c < columns; c += 32) {
+        float sum = 0.0f;
+        for (int b = b0; b < b1; ++b)
+            if (gb_odd_half(*reinterpret_cast<const unsigned short *>(wrow + (int64_t)b * BB)))
+                sum += gb_term<QT>(wrow + (int64_t)b * BB, p.x + (int64_t)(c0 + c) * p.ldx + (int64_t)b * kQK, p.order);
+        out[c * ld] = (p.xscale[c0 + c] < 0.0f ? out[c * ld] : bias ? p.bias[j] : 0.0f) + sum;
+    }
+}
+// Whether any of the 256 epilogue threads says so.
+__device__ __forceinline__ bool gb_any(bool mine) {
+    int any;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbarrier.cta.red.or.pred q, 1, 256, p;\n\tselp.s32 %0, 1, 0, q;\n\t}" : "=r"(any) : "r"((int)mine) : "memory");
+    return any;
 }
 
 template <int R>
@@ -217,7 +285,7 @@ __device__ __forceinline__ uint64_t smem_desc_k64(uint32_t smem_addr) {
 
 template <int QT, int NB>
 __global__ void __launch_bounds__(GbCfg<QT, NB>::kThreads, 1)
-    gemm_blocks_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmFix, const GpParams p) {
+    gemm_blocks_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmFix, const __grid_constant__ GpParams p) {
     using Cfg = GbCfg<QT, NB>;
     constexpr int WST = Cfg::kWStages, XST = Cfg::kXStages, ROWCHUNK = Cfg::kRowChunk;
     constexpr int BPS = 128 / NB;  // blocks per slot: 1, 2
@@ -256,11 +324,11 @@ __global__ void __launch_bounds__(GbCfg<QT, NB>::kThreads, 1)
         fence_mbar_init();
     }
     if constexpr (Cfg::kFix) {
-        // Row r of the K-major tile: K = 16 step j (16-byte pieces 2j, 2j + 1, at piece ^ (r & 7)) has 512 at 2j, 2j + 1.
+        // Row r of the K-major tile: K = 16 step j (16-byte pieces 2j, 2j + 1, at piece ^ (r & 7)) has 512 at 2j, 512 * 2^-11 at 2j + 1.
         for (int i = threadIdx.x; i < GP_ROWS * 8; i += Cfg::kThreads) {
             const int r = i >> 3, piece = i & 7, j = piece >> 1;
             uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if ((piece & 1) == 0) (j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w) = 0x60006000u;
+            if ((piece & 1) == 0) (j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w) = 0x34006000u;
             *reinterpret_cast<uint4 *>(smem_ones + r * 128 + ((piece ^ (r & 7)) << 4)) = v;
         }
     }
@@ -359,10 +427,13 @@ __global__ void __launch_bounds__(GbCfg<QT, NB>::kThreads, 1)
                             const uint32_t acc = tmem_base + (uint32_t)(slot * 128 + (BPS == 1 ? 0 : blk * NB));
                             tc_mma_f16_ts(acc, ah + 16 * blk, xl + 4 * blk, idesc, 0);
                             tc_mma_f16_ts(acc, ah + 16 * blk + 8, xl + 4 * blk + 2, idesc, 1);
-                            if constexpr (Cfg::kFix)
-                                tc_mma_f16(acc, smem_desc_k128(smem_u32(smem_ones)) + (uint64_t)(2 * (2 * (u & 1) + blk)),
-                                           smem_desc_k64(smem_u32(smem_fix + ((u >> 2) & 1) * Cfg::kFixBytes)) + (uint64_t)(2 * ((u >> 1) & 1)), idesc, 1);
-                            tc_mma_f16_ts(acc, ah + 16 * blk, xh + 4 * blk, idesc, 1);
+                            if constexpr (Cfg::kFix) {
+                                tc_mma_f16_scaled<GB_LO_BITS>(acc, smem_desc_k128(smem_u32(smem_ones)) + (uint64_t)(2 * (2 * (u & 1) + blk)),
+                                                              smem_desc_k64(smem_u32(smem_fix + ((u >> 2) & 1) * Cfg::kFixBytes)) + (uint64_t)(2 * ((u >> 1) & 1)), idesc);
+                                tc_mma_f16_ts(acc, ah + 16 * blk, xh + 4 * blk, idesc, 1);
+                            } else {
+                                tc_mma_f16_ts_scaled<GB_LO_BITS>(acc, ah + 16 * blk, xh + 4 * blk, idesc);
+                            }
                             tc_mma_f16_ts(acc, ah + 16 * blk + 8, xh + 4 * blk + 2, idesc, 1);
                             if (ends) {
                                 tc_commit(smem_u32(&d_full[slot]));
@@ -461,7 +532,7 @@ __global__ void __launch_bounds__(GbCfg<QT, NB>::kThreads, 1)
         const uint32_t from = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(part * COLS);
         const int first_tile = g0 / p.nchunks;
         int u = 0, slot = 0, use = 0;
-        bool ok = true;
+        bool ok = true, odd = false, hurt = false;  // (rows that the tensor core does not take, of either operand)
         for (int g = g0; g < g1 && ok;) {
             const int tile = g / p.nchunks, c0 = g - tile * p.nchunks, cn = min(p.nchunks - c0, g1 - g);
             g += cn;
@@ -469,7 +540,6 @@ __global__ void __launch_bounds__(GbCfg<QT, NB>::kThreads, 1)
             uint64_t acc[COLS / 2];
 #pragma unroll
             for (int j = 0; j < COLS / 2; ++j) acc[j] = 0;
-            bool mine = false;  // a scale that is not finite
             for (int e = u + 4 * cn; u < e && ok; ++u) {
                 uint32_t two = 0;
 #pragma unroll
@@ -490,7 +560,7 @@ __global__ void __launch_bounds__(GbCfg<QT, NB>::kThreads, 1)
                         const int blk = gq * BPS + b;
                         if (blk == 0) {
                             asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(two) : "r"(smem_u32(&smem_d[(u & (GB_SCALES - 1)) * GP_ROWS + r])) : "memory");
-                            mine |= (((two & 0x7C007C00u) + 0x04000400u) & 0x80008000u) != 0;
+                            hurt |= (((two & 0x7C007C00u) + 0x04000400u) & 0x80008000u) != 0;
                         }
                         d[b] = __half2float(__ushort_as_half((unsigned short)(blk ? two >> 16 : two & 0xFFFFu)));
                     }
@@ -517,25 +587,42 @@ __global__ void __launch_bounds__(GbCfg<QT, NB>::kThreads, 1)
             float scales[COLS / 32];
 #pragma unroll
             for (int j = 0; j < COLS / 32; ++j) scales[j] = p.xscale[min(col0 + 32 * j + lane, p.m - 1)];
-            bool low = false;
 #pragma unroll
             for (int j = 0; j < COLS / 2; ++j) {
                 const float s0 = __shfl_sync(0xffffffffu, scales[j / 16], (2 * j) & 31), s1 = __shfl_sync(0xffffffffu, scales[j / 16], (2 * j + 1) & 31);
                 float v0, v1;
                 unpack2(acc[j], v0, v1);
-                low |= s0 < 0.0f || s1 < 0.0f;
+                odd |= s0 < 0.0f || s1 < 0.0f;
                 if (row < p.n) {
                     if (col0 + 2 * j < p.m) dst[(int64_t)(2 * j) * ld] = fmaf(v0, s0, bias);
                     if (col0 + 2 * j + 1 < p.m) dst[(int64_t)(2 * j + 1) * ld] = fmaf(v1, s1, bias);
                 }
             }
-            if ((mine || low) && row < p.n) {
-                for (int c = 0; c < COLS && col0 + c < p.m; ++c)
-                    if (mine || p.xscale[col0 + c] < 0.0f)
-                        dst[c * ld] = bias + gb_plain_dot<QT>(p.w + (int64_t)row * (p.k / kQK) * Cfg::kBlockBytes, p.x + (int64_t)(col0 + c) * p.ldx, p.order,
-                                                                  c0 * 8, (c0 + cn) * 8);
-            }
             __syncwarp();
+        }
+        // All units are done with, the slabs of X among them.  (Every one of the 256 threads takes the same way from here.)
+        if (gb_any(odd || hurt || !ok) && !gb_any(!ok)) {
+            const bool some_hurt = gb_any(hurt);
+            const int t = threadIdx.x - 32 * Cfg::kWarpEp0;
+            for (int g = g0; g < g1;) {
+                const int tile = g / p.nchunks, c0 = g - tile * p.nchunks, cn = min(p.nchunks - c0, g1 - g), b0 = c0 * 8, b1 = (c0 + cn) * 8;
+                g += cn;
+                const int group = tile / p.mtiles, col0 = (tile - group * p.mtiles) * NB, j0 = group * GP_ROWS, columns = min(NB, p.m - col0);
+                const bool direct = cn == p.nchunks;
+                const int64_t ld = direct ? p.ldy : GP_ROWS;
+                float *out = direct ? p.y + (int64_t)col0 * p.ldy + j0 : p.part + (int64_t)(2 * blockIdx.x + (tile == first_tile ? 0 : 1)) * NB * GP_ROWS;
+                for (int c = 0; c < columns; ++c)
+                    if (p.xscale[col0 + c] < 0.0f) gb_odd_row<QT>(p, j0, col0 + c, b0, b1, reinterpret_cast<int *>(smem_x), out + c * ld, direct && p.bias, t);
+                if (some_hurt) {
+                    asm volatile("barrier.cta.sync 1, 256;" ::: "memory");  // the batch rows' sums are there to be added to
+                    for (int r = t >> 5; r < GP_ROWS && j0 + r < p.n; r += 8) {
+                        bool bad = false;
+                        for (int b = b0 + lane; b < b1; b += 32)
+                            bad |= gb_odd_half(*reinterpret_cast<const unsigned short *>(p.w + ((int64_t)(j0 + r) * (p.k / kQK) + b) * Cfg::kBlockBytes));
+                        if (__any_sync(0xffffffffu, bad)) gb_odd_weights<QT>(p, j0 + r, col0, columns, b0, b1, out + r, ld, direct && p.bias, lane);
+                    }
+                }
+            }
         }
     }
     tc_fence_before();

@@ -83,8 +83,37 @@ def test_operands_outside_f16(device, qt, order):
     t[:, 299] = terms(qt, order, np.nan_to_num(x, posinf=0.0), hurt[299:].reshape(-1), 1)[:, 0]
     bound = (k // 32 + 4) * 2.0 ** -23 * t + 2.0 ** -23 * np.abs(want)
     assert (np.abs(y - want)[f] <= bound[f]).all()
-    # the small blocks themselves, through weights that see nothing else
+
+
+@pytest.mark.parametrize("qt,order", QT_ORDERS)
+@pytest.mark.parametrize("m,k", [(40, 512), (128, 28672)])
+def test_small_blocks_beside_large_ones(device, qt, order, m, k):
+    """Blocks of 2^0 .. 2^-12 in rows whose others reach 2^12 (Q4_0, whose blocks' sums f16 has to hold) or 2^20, through weights
+    that see nothing else: a block's own product is exact, so d8 and two roundings in f32 are all that there is.  And with all
+    weights, every row of the batch like that, 28672 values long."""
+    n = 260
+    rng = np.random.default_rng(k + qt + order)
+    blocks = oc.quantize(qt, order, (rng.standard_normal((n, k)) * 0.02).astype(np.float32)).reshape(n, k // 32, -1)
+    x = (rng.standard_normal((m, k)) * (2.0 ** 10 if qt == oc.Q4_0 else 2.0 ** 20)).astype(np.float32)
+    x[:, 64:96] = rng.standard_normal((m, 32)) * 2.0 ** -(np.arange(m) % 13)[:, None]
     only = np.zeros_like(blocks)
     only[:, 2] = blocks[:, 2]
-    y, want = (call(device, qt, order, np.repeat(x[1:3], 20, 0), only.reshape(-1), n, integer=i) for i in (False, True))
-    assert np.linalg.norm(y - want) <= 1e-6 * np.linalg.norm(want)
+    y, want = (call(device, qt, order, x, only.reshape(-1), n, integer=i) for i in (False, True))
+    assert (np.abs(want).max(1) > 0.0).all()
+    assert (np.linalg.norm(y - want, axis=1) <= 2.0 ** -21 * np.linalg.norm(want, axis=1)).all()
+    y, want = (call(device, qt, order, x, blocks.reshape(-1), n, integer=i) for i in (False, True))
+    assert (np.abs(y - want) <= (k // 32 + 4) * 2.0 ** -23 * terms(qt, order, x, blocks, n) + 2.0 ** -23 * np.abs(want)).all()
+
+
+@pytest.mark.parametrize("qt,order", QT_ORDERS)
+def test_every_row_outside_f16(device, qt, order):
+    """A d8 or s8 in every row of a full tile that f16 does not hold, in several pieces of k: the infinities of
+    the integer dots, and nothing that any wait in the kernel runs out over."""
+    m, n, k = 128, 300, 40960
+    rng = np.random.default_rng(order)
+    blocks = oc.quantize(qt, order, (rng.standard_normal((n, k)) * 0.02).astype(np.float32))
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    x[np.arange(m), rng.integers(0, k, m)] = np.where(np.arange(m) % 2, 9e6, -9e6)
+    y, want = (call(device, qt, order, x, blocks, n, integer=i) for i in (False, True))
+    assert np.array_equal(np.isnan(y), np.isnan(want)) and np.array_equal(y[np.isinf(want)], want[np.isinf(want)])
+    assert not np.isfinite(y).any() and not np.isfinite(want).any()

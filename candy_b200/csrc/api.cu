@@ -453,9 +453,11 @@ cq_status cq_qmatmul(cq_ctx *ctx, int qtype, int order, int actmode, const float
         // captured without the scratch for its operands (4 m k bytes), or no memory for it: the planes below do with about half
         if (!(s == CQ_ERR_INVALID_ARG && cq_stream_capturing(ctx)) && s != CQ_ERR_NOMEM) return s;
     }
-    // CQ_ACT_Q8_1 from 33 rows on: the same with one product per weight block, scaled in f32 (us, integer dots below in brackets:
-    // n 11008 x k 4096, Q4_0 / Q8_0, 33 rows 32 (44) / 29 (36), 100 rows 39 (73) / 39 (64), 300 rows 85 (217) / 81 (188); 700 x
-    // 1024, 33 rows 12.2 (13.2) / 11.2 (11.5).  32 rows are even there, 30 (31) / 26.5 (27.6), but 4096 x 14336 43 (39) / 38 (33).)
+    // CQ_ACT_Q8_1 from 33 rows on: the same with one product per weight block, scaled in f32.  us, Q4_0 / Q8_0, the integer dots
+    // below in brackets, back to back calls on weights that stay in L2: n 11008 x k 4096, 33 rows 31 (43) / 29 (35), 100 rows 39 (73)
+    // / 37 (63); 4096 x 14336, 33 rows 41 (54) / 37 (44); 1024 x 14336, 40 rows 21 (26) / 20 (23), 33 rows 25 (25) / 23 (22); 700 x
+    // 1024, 33 rows 12.5 (13.2) / 11.9 (11.6).  At 32 rows, where the integer kernel has half the columns, it is the quicker one on
+    // long rows: 4096 x 14336 38 / 32 against 41 / 37.
     if (actmode == CQ_ACT_Q8_1 && ctx->tune.split_min_rows_q8_1 > 0 && m >= ctx->tune.split_min_rows_q8_1 && on_f16_sums) {
         s = launch_gemm_blocks(ctx, qtype, order, x_dev, m, k, ldx, w_blocks_dev, n, y_dev, ldy);
         // (captured without the scratch for its operands, no memory for them, or too many tiles in one launch: the integer dots)

@@ -80,36 +80,39 @@ __device__ __forceinline__ float gb_q8(float v, float d) { return (float)(int)ro
 // multiple of 2^-21; a d8 below f16's normal numbers is up to twice amax / 127 and leaves hi below 65024 and lo 2^11 below 2^15.
 // A row with a d8 or s8 that is not finite gets a negative scale, which leaves it to the epilogue warps.
 // fix: [m][k / 8], per 128 k the four blocks' (c_hi, c_lo 2^11) and eight zeros.
-__global__ void __launch_bounds__(256) gb_x_q8_kernel(const float *__restrict__ x, int64_t k, int64_t ldx, int order, __half *__restrict__ hi,
+__global__ void __launch_bounds__(1024) gb_x_q8_kernel(const float *__restrict__ x, int64_t k, int64_t ldx, int order, __half *__restrict__ hi,
                                                        __half *__restrict__ lo, __half *__restrict__ fix, float *__restrict__ scale) {
     pdl_launch_dependents();
     pdl_wait_prior();
-    __shared__ float red[8];
+    __shared__ float red[32];
+    const int threads = blockDim.x;
     const int64_t row = blockIdx.x;
     const float *src = x + row * ldx;
     const bool vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0 && ldx % 4 == 0;
     float amax = 0.0f;
     if (vec) {
-        for (int64_t i = threadIdx.x; i < k / 4; i += 256) {
+#pragma unroll 4
+        for (int64_t i = threadIdx.x; i < k / 4; i += threads) {
             const float4 t = reinterpret_cast<const float4 *>(src)[i];
             amax = fmaxf(amax, fmaxf(fmaxf(fabsf(t.x), fabsf(t.y)), fmaxf(fabsf(t.z), fabsf(t.w))));
         }
     } else {
-        for (int64_t i = threadIdx.x; i < k; i += 256) amax = fmaxf(amax, fabsf(src[i]));
+        for (int64_t i = threadIdx.x; i < k; i += threads) amax = fmaxf(amax, fabsf(src[i]));
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
     __syncthreads();
     amax = red[0];
+    for (int i = 0; i < threads / 32; i += 8)
 #pragma unroll
-    for (int i = 1; i < 8; ++i) amax = fmaxf(amax, red[i]);
+        for (int j = 0; j < 8; ++j) amax = fmaxf(amax, red[i + j]);
     int e = 0;
     if (amax > 0.0f && amax < INFINITY) e = min(14 - ilogbf(amax), 126);
     const float up = __int_as_float((127 + e) << 23);  // e in [-113, 126]
     bool odd = false;
 #pragma unroll 4
-    for (int64_t o8 = threadIdx.x; o8 < k / 8; o8 += 256) {
+    for (int64_t o8 = threadIdx.x; o8 < k / 8; o8 += threads) {
         float v[8];
         load_permuted8(src + (o8 >> 2) * 32, (int)(o8 & 3), order, vec, v);
         // a block's 32 values lie in four neighbouring lanes (k is a multiple of 256: warps are in the loop as a whole)
@@ -676,7 +679,11 @@ cq_status gb_run(cq_ctx *ctx, const float *x, int64_t m, int64_t k, int64_t ldx,
     if (!gp_w_map(&tmW, w, n, (k / kQK) * Cfg::kBlockBytes, Cfg::kRowChunk) || !gp_x_map(&tmX, xh, m, k, x_bytes, NB, 1) ||
         (Cfg::kFix && !gb_fix_map(&tmFix, fix, m, k, NB)))
         return cq_fail(ctx, CQ_ERR_CUDA, "gemm: cuTensorMapEncodeTiled failed or is unavailable");
-    s = gp_launch(ctx, gb_x_q8_kernel, dim3((unsigned)m), 256, 0, false, x, k, ldx, QT == CQ_Q4_0 ? order : 2, xh, xl, fix, scale);
+    // Threads per row of the pre-pass: where its CTAs have an SM each or share it with one other, a long row wants more than 256.
+    // (us of the call at n 700, Q4_0, 256 / 512 / 1024 threads: 64 rows of 4096 values 15.5 / 14.7 / 14.0, of 14336 32.4 / 27.1 /
+    // 21.4; 200 rows of 2048 18.2 / 16.5 / 19.6, of 14336 39.9 / 37.6 / 39.5; 400 rows of 4096 27.7 / 29.1 / 32.3.)
+    const int threads = m <= ctx->sm_count && k >= 8192 ? 1024 : (m <= 2 * ctx->sm_count && k >= 2048 ? 512 : 256);
+    s = gp_launch(ctx, gb_x_q8_kernel, dim3((unsigned)m), threads, 0, false, x, k, ldx, QT == CQ_Q4_0 ? order : 2, xh, xl, fix, scale);
     if (s == CQ_OK) s = gp_launch(ctx, kern, dim3(sh.shares), Cfg::kThreads, Cfg::kSmem, false, tmW, tmX, tmFix, p);
     if (s == CQ_OK && sh.cut) s = gp_launch(ctx, gp_sum_kernel<GP_ROWS, NB>, dim3((unsigned)sh.tiles, NB / 8), 256, 0, false, p);
     if (s == CQ_OK && p.bias) ctx->bias_done = true;

@@ -608,12 +608,18 @@ __global__ void __launch_bounds__(128) attn_partial_gqa_kernel(const float *__re
 // every lane its own dims): 8 to 12 KB a warp, sixteen warps an SM.
 // Bound: HBM (f32 caches, read once for all G heads).  The kernel before this one staged K and V in shared memory for the four
 // warps together, and read q and p from there, the same words for every lane: 2200 cycles of shared-memory bandwidth and three
-// barriers per 64 keys.  64 / 8 heads, 32 sequences x 2048 keys, us: before 140, now 108, floor 82;
-// 2 x 64 / 8 heads x 16384 72 -> 61, one sequence of 2048 keys 11.7 -> 12.4.
+// barriers per 64 keys.  64 / 8 heads, a call with its combining launch, caches from HBM, us, that kernel -> this one (floor: the
+// caches' bytes): 32 sequences x 2048 keys 199 -> 107 (82), 8 x 2048 67 -> 38 (20), 1 x 2048 12.8 -> 12.6 (2.6), 1 x 1024 11.5 -> 9.9,
+// 2 x 16384 105 -> 66 (41).  What the short ones need (1 x 2048 was 17 without): the loads of all heads' q together 1.2 us, an even
+// number of CTAs on every SM 2.4, the combining's first loads beside its weights 0.4, K's next lines on their way to L2 0.3.
 // Writes (max, sum, acc[128]) per (head, split) in the layout the combine kernel reads.
 constexpr int kAttn2Keys = 32;  // keys that a CTA takes per round: splits are multiples of it
 constexpr int kAttn2Stages = 3; // rounds of V in shared memory
 constexpr size_t kAttn2Smem = (size_t)4 * kAttn2Stages * 8 * 128 * 4;  // [warp][round][key][dim]; at the end the warps' sums
+// What a launch asks for whose CTAs make 1, 2, 3, 4 or more per SM: no SM can take more than that.  Launched behind a kernel that is still
+// finishing, CTAs pile up on the SMs that are free first, and a few SMs set the time (us of 16 sequences x 8 kv heads x 2048 keys
+// in one split, 128 CTAs: 157, with an SM each 100; one sequence in 32 splits 16.7 and 14.2).
+constexpr size_t kAttn2SmemOf[4] = {200 << 10, 100 << 10, 66 << 10, kAttn2Smem};
 template <bool ROPE>
 __global__ void __launch_bounds__(128, 4) attn_split_gqa_kernel(const float *__restrict__ qkv, int nq, int nkv, const int *__restrict__ pos_dev,
                                                               const float *kc, const float *vc, int max_ctx, float scale, float *__restrict__ part,
@@ -693,6 +699,11 @@ __global__ void __launch_bounds__(128, 4) attn_split_gqa_kernel(const float *__r
         }
     };
     auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
+    // A warp's next eight keys on their way to L2, a 128-byte line a lane: the loads of K reach one round ahead only.
+    auto prefetch_k = [&](int t) {
+        const float *line = kc + ((int64_t)b * max_ctx + min(t + (lane >> 2), t_end - 1)) * kv_stride + kvh * hd + 32 * (lane & 3);
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(line));
+    };
     float m_run = kLow, l_run = 0.0f;  // of head c: its maximum so far, and this lane's part of its sum
     float4 kr[2][4];
     int t = t_begin + 8 * warp, stage = 0;
@@ -701,16 +712,26 @@ __global__ void __launch_bounds__(128, 4) attn_split_gqa_kernel(const float *__r
         fetch_v(t, 0);
     }
     commit();
-    if (t + 32 < t_end) fetch_v(t + 32, 1);
+    if (t + 32 < t_end) {
+        prefetch_k(t + 32);
+        fetch_v(t + 32, 1);
+    }
     commit();
     // q of the group's heads (rotated here when the rotary step is fused in: cos_t given), while the first keys are on their way
-    for (int i = tid; i < 8 * hd; i += 128) {
-        const float *qh = qkv + (int64_t)b * row + (kvh * G + i / hd) * hd;
-        q_s[i / hd][i % hd] = (i / hd) < G ? (ROPE ? rope_elem(qh, i % hd, hd, cos_t, sin_t, nkeys - 1) : qh[i % hd]) : 0.0f;
+    float q_new[8];  // (all heads' loads together)
+#pragma unroll
+    for (int g = 0; g < 8; ++g) {
+        const float *qh = qkv + (int64_t)b * row + (kvh * G + min(g, G - 1)) * hd;
+        q_new[g] = ROPE ? rope_elem(qh, tid, hd, cos_t, sin_t, nkeys - 1) : qh[tid];
     }
+#pragma unroll
+    for (int g = 0; g < 8; ++g) q_s[g][tid] = g < G ? q_new[g] : 0.0f;
     __syncthreads();
     for (; t < t_end; t += 32) {
-        if (t + 64 < t_end) fetch_v(t + 64, stage == 0 ? 2 : stage - 1);
+        if (t + 64 < t_end) {
+            prefetch_k(t + 64);
+            fetch_v(t + 64, stage == 0 ? 2 : stage - 1);
+        }
         commit();
         float s[2][8];
 #pragma unroll
@@ -800,41 +821,56 @@ __global__ void __launch_bounds__(128, 4) attn_split_gqa_kernel(const float *__r
 }
 
 // Combines the chunk partials of one (head, sequence): out[b][head*hd + d].  Lane = four
-// consecutive dims, the four warps take every fourth chunk; all loads of a batch of eight chunks
-// are unconditional (clamped index, zero weight past the end) so they are in flight together.
-__global__ void __launch_bounds__(128) attn_combine_kernel(const float *__restrict__ part, int nq, int hd, int nchunks,
-                                                         float *__restrict__ out) {
+// consecutive dims, the warps take every WARPS-th chunk; all loads of a batch of eight chunks
+// are unconditional (clamped index, zero weight past the end) so they are in flight together, the
+// first batch's with the maxima and sums (weights come after).  Eight warps where grouped heads have
+// more than 32 splits, which is then one batch.
+template <int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) attn_combine_kernel(const float *__restrict__ part, int nq, int hd, int nchunks,
+                                                                float *__restrict__ out) {
     __shared__ float w_s[512];  // per-chunk weight exp(m_c - m); nchunks <= 512 (context <= 16384)
     __shared__ float red[32];
-    __shared__ float4 acc_s[4][64];  // per-warp partial sums, hd <= 256
+    __shared__ float4 acc_s[WARPS][64];  // per-warp partial sums, hd <= 256
     pdl_launch_dependents();
     pdl_wait_prior();
     const int head = blockIdx.x, b = blockIdx.y;
     const int stride = hd + 2;
     const float *p = part + (((int64_t)b * nq + head) * nchunks) * stride;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // chunk maxima and sums: one (m, l) pair per thread per trip, both loads issued together
     float m = -3.402823466e38f;
-    float mc[4], lc[4];
+    constexpr int TRIPS = 16 / WARPS;
+    float mc[TRIPS], lc[TRIPS];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int c = threadIdx.x + i * 128;
+    for (int i = 0; i < TRIPS; ++i) {
+        const int c = threadIdx.x + i * 32 * WARPS;
         const int cc = c < nchunks ? c : nchunks - 1;
         mc[i] = p[(int64_t)cc * stride];
         lc[i] = p[(int64_t)cc * stride + 1];
         if (c >= nchunks) mc[i] = -3.402823466e38f, lc[i] = 0.0f;
-        m = fmaxf(m, mc[i]);
     }
+    float a[8][4];
+    auto load = [&](int c0, int d) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float *q = p + 2 + (d < hd ? d : 0) + (int64_t)min(c0 + WARPS * j, nchunks - 1) * stride;  // rows start 8 bytes past a 16-byte boundary: two 8-byte loads
+            const float2 lo = *reinterpret_cast<const float2 *>(q), hi = *reinterpret_cast<const float2 *>(q + 2);
+            a[j][0] = lo.x, a[j][1] = lo.y, a[j][2] = hi.x, a[j][3] = hi.y;
+        }
+    };
+    load(warp, lane * 4);
+#pragma unroll
+    for (int i = 0; i < TRIPS; ++i) m = fmaxf(m, mc[i]);
     m = warp_max(m);
     if (lane == 0) red[warp] = m;
     __syncthreads();
-    m = (lane < nw) ? red[lane] : -3.402823466e38f;
+    m = (lane < WARPS) ? red[lane] : -3.402823466e38f;
     m = warp_max(m);
     __syncthreads();
     float l = 0.0f;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int c = threadIdx.x + i * 128;
+    for (int i = 0; i < TRIPS; ++i) {
+        const int c = threadIdx.x + i * 32 * WARPS;
         const float w = (c < nchunks) ? expf(mc[i] - m) : 0.0f;
         if (c < nchunks) w_s[c] = w;
         l = fmaf(w, lc[i], l);
@@ -842,36 +878,26 @@ __global__ void __launch_bounds__(128) attn_combine_kernel(const float *__restri
     l = block_sum(l, red);  // has the barriers that publish w_s
     const float inv = 1.0f / l;
     for (int d0 = 0; d0 < hd; d0 += 128) {
-        const int d = d0 + lane * 4;
-        const bool live = d < hd;
-        const float *pd = p + 2 + (live ? d : 0);
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int c0 = warp; c0 < nchunks; c0 += 32) {
-            float a[8][4];
-            float w[8];
+        for (int c0 = warp; c0 < nchunks; c0 += 8 * WARPS) {
+            if (c0 != warp || d0 != 0) load(c0, d0 + lane * 4);
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                const int c = c0 + 4 * j;
-                const int cc = c < nchunks ? c : nchunks - 1;
-                const float *q = pd + (int64_t)cc * stride;  // rows start 8 bytes past a 16-byte boundary: two 8-byte loads
-                const float2 lo = *reinterpret_cast<const float2 *>(q), hi = *reinterpret_cast<const float2 *>(q + 2);
-                a[j][0] = lo.x, a[j][1] = lo.y, a[j][2] = hi.x, a[j][3] = hi.y;
-                w[j] = c < nchunks ? w_s[c] : 0.0f;
-            }
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                acc.x = fmaf(a[j][0], w[j], acc.x);
-                acc.y = fmaf(a[j][1], w[j], acc.y);
-                acc.z = fmaf(a[j][2], w[j], acc.z);
-                acc.w = fmaf(a[j][3], w[j], acc.w);
+                const int c = c0 + WARPS * j;
+                const float w = c < nchunks ? w_s[c] : 0.0f;
+                acc.x = fmaf(a[j][0], w, acc.x);
+                acc.y = fmaf(a[j][1], w, acc.y);
+                acc.z = fmaf(a[j][2], w, acc.z);
+                acc.w = fmaf(a[j][3], w, acc.w);
             }
         }
         acc_s[warp][(d0 >> 2) + lane] = acc;
     }
     __syncthreads();
-    for (int d = threadIdx.x; d < hd; d += blockDim.x) {
+    for (int d = threadIdx.x; d < hd; d += 32 * WARPS) {
         const float *f = reinterpret_cast<const float *>(&acc_s[0][0]);
-        const float v = (f[d] + f[256 + d]) + (f[512 + d] + f[768 + d]);
+        float v = (f[d] + f[256 + d]) + (f[512 + d] + f[768 + d]);
+        if constexpr (WARPS == 8) v += (f[1024 + d] + f[1280 + d]) + (f[1536 + d] + f[1792 + d]);
         out[((int64_t)b * nq + head) * hd + d] = v * inv;
     }
 }
@@ -1174,26 +1200,33 @@ cq_status attention_impl(cq_ctx *ctx, float *qkv_dev, int64_t batch, int n_q_hea
         return CQ_OK;
     }
     if (split_route) {
-        // Splits of the keys: what a round of CTAs (four per SM) takes at the longest context, its keys and about 96 keys' worth of
-        // start and end, times the rounds, and two keys' worth per split for combining.  (us with 1, 2, 4, 8, 16, 32, 64 splits: 32
-        // sequences x 8 kv heads x 2048 keys 177, 108, 103, 111, 129, 163, 235; 4 x 8 x 2048 68, 37, 34, 22, 18.5, 21, 26; 1 x 8 x 2048
-        // 67, 36, 22, 14.5, 13.3, 12.4, 13.4; 2 x 8 x 16384 492, 254, 134, 114, 69, 61, 66; 1 x 8 x 128 9.4, 7.7, 6.7.)
-        const int64_t pairs = (int64_t)n_kv_heads * batch, slots = (int64_t)ctx->sm_count * 4;
+        // Splits of the keys at the longest context, by what an SM has to do: `per` CTAs, each with `keys` keys, that hide each
+        // other's latencies the better the more there are (up to four at a time); 37 keys' worth to start and end a CTA, 105 for each
+        // four; two for a split's part of the combining.  Fitted to 33 shapes, 1 to 48 sequences of 128 to 16384 keys with 2 to 8 heads a
+        // group: the split taken is 1 % slower than the best one on average, 9 % at most.  (us with 1, 2, 4, 8, 16, 32, 64 splits, the
+        // one taken in brackets: 1 sequence x 8 kv heads x 2048 keys -, -, 29.5, 18.5, 13.5, [12.6], 12.4; 4 x 8 x 2048 97, 53, 31,
+        // [25.3], 25.2, 28, 34; 8 x 8 x 2048 99, 55, 41, 38, 42, 45, 55 [6 splits: 38.0]; 16 x 8 x 2048 100, 70, 63, [64], 70, 80, 103;
+        // 32 x 8 x 2048 129, 112, [107], 116, 132, 155, 199; 2 x 8 x 16384 -, 366, 187, 99, 68, 61, 63 [27: 66].)
+        const int64_t pairs = (int64_t)n_kv_heads * batch;
         int64_t best = INT64_MAX;
         for (int i = 1, most = std::min(nchunks, 64); i <= most; ++i) {  // (a chunk of scratch is 32 keys)
-            const int64_t cost = (pairs * i + slots - 1) / slots * ((max_ctx + i - 1) / i + 96) + 2 * i;
+            const int keys = ((max_ctx + i - 1) / i + kAttn2Keys - 1) / kAttn2Keys * kAttn2Keys;
+            if ((max_ctx + keys - 1) / keys != i) continue;  // the last ones would have no keys
+            static constexpr int kPercent[4] = {178, 117, 115, 100};
+            const int64_t per = (pairs * i + ctx->sm_count - 1) / ctx->sm_count;
+            const int64_t cost = per * keys * kPercent[std::min<int64_t>(per, 4) - 1] / 100 + 37 * per + 105 * ((per + 3) / 4) + 2 * i;
             if (cost < best) best = cost, nchunks = i;
         }
         static thread_local int configured = -1;
         if (configured != ctx->device) {
-            CQ_CUDA(ctx, cudaFuncSetAttribute(attn_split_gqa_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAttn2Smem));
-            CQ_CUDA(ctx, cudaFuncSetAttribute(attn_split_gqa_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAttn2Smem));
+            CQ_CUDA(ctx, cudaFuncSetAttribute(attn_split_gqa_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAttn2SmemOf[0]));
+            CQ_CUDA(ctx, cudaFuncSetAttribute(attn_split_gqa_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAttn2SmemOf[0]));
             configured = ctx->device;
         }
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)nchunks, (unsigned)n_kv_heads, (unsigned)batch);
         cfg.blockDim = dim3(128);
-        cfg.dynamicSmemBytes = kAttn2Smem;
+        cfg.dynamicSmemBytes = kAttn2SmemOf[std::min<int64_t>(4, (pairs * nchunks + ctx->sm_count - 1) / ctx->sm_count) - 1];
         cfg.stream = ctx->stream;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1217,7 +1250,10 @@ cq_status attention_impl(cq_ctx *ctx, float *qkv_dev, int64_t batch, int n_q_hea
                        (const float *)qkv_dev, n_q_heads, n_kv_heads, head_dim, pos_dev, (const float *)k_cache_dev, (const float *)v_cache_dev, max_ctx,
                        scale, scratch_dev, nchunks, cos_dev, sin_dev, k_cache_dev, v_cache_dev, ctx->dev_err_devptr);
     if (s != CQ_OK) return s;
-    return launch_pdl(ctx, attn_combine_kernel, dim3((unsigned)n_q_heads, (unsigned)batch), dim3(128), (const float *)scratch_dev, n_q_heads,
+    if (split_route && nchunks > 32)
+        return launch_pdl(ctx, attn_combine_kernel<8>, dim3((unsigned)n_q_heads, (unsigned)batch), dim3(256), (const float *)scratch_dev, n_q_heads,
+                          head_dim, nchunks, out_dev);
+    return launch_pdl(ctx, attn_combine_kernel<4>, dim3((unsigned)n_q_heads, (unsigned)batch), dim3(128), (const float *)scratch_dev, n_q_heads,
                       head_dim, nchunks, out_dev);
 }
 }  // namespace

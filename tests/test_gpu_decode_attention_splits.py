@@ -12,6 +12,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("rope", [False, True])
 @pytest.mark.parametrize("batch,nkv,G,max_ctx,positions", [
     (1, 1, 2, 40, (0, 6, 7, 8, 9)), (2, 2, 3, 200, (30, 31, 32, 33, 199)), (1, 4, 8, 520, (63, 64, 255, 519)), (3, 2, 5, 70, (1, 69)), (40, 8, 4, 100, (99,)),
+    (1, 2, 2, 4100, (0, 40, 1500, 4099)), (20, 8, 2, 150, (0, 149)),
 ])
 def test_rounds_and_splits(device, batch, nkv, G, max_ctx, positions, rope):
     lib, ctx, hd = device._lib, device.ctx, 128

@@ -1,11 +1,13 @@
 """CQ_ACT_Q8_1 batches of 33 rows and more (f16 products per weight block, scaled in f32): the edges of its tiles (128 weight
 rows, 64 / 128 batch rows, chunks of 256 k, shares that cut a tile) against the oracle of the reference's CUDA arithmetic, and
 operands that the tensor core does not take against the integer dots of smaller batches."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
 from candy_b200 import abi
-from candy_b200.backend import ACT_Q8_1, QStorage
+from candy_b200.backend import ACT_Q8_1, CudaDevice, QStorage
 from oracle import oracle_c as oc
 
 pytestmark = pytest.mark.gpu
@@ -117,3 +119,38 @@ def test_every_row_outside_f16(device, qt, order):
     y, want = (call(device, qt, order, x, blocks, n, integer=i) for i in (False, True))
     assert np.array_equal(np.isnan(y), np.isnan(want)) and np.array_equal(y[np.isinf(want)], want[np.isinf(want)])
     assert not np.isfinite(y).any() and not np.isfinite(want).any()
+
+
+@pytest.mark.parametrize("qt", [oc.Q4_0, oc.Q8_0])
+@pytest.mark.parametrize("m,n,k,room", [
+    (1000, 300, 8192, lambda m, k: 5 * m * k // 4 + (20 << 20)),                      # what the integer dots need: they serve it
+    (100, 2000, 4096, lambda m, k: 4 * m * k + m * k // 4 + 4 * m + (4 << 10)),       # the operands, no partial tiles: whole tiles
+])
+def test_captured_with_little_scratch(qt, m, n, k, room):
+    dev = CudaDevice(0)
+    rng = np.random.default_rng(m)
+    blocks = oc.quantize(qt, 0, (rng.standard_normal((n, k)) * 0.02).astype(np.float32))
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    qs, xd, yd = QStorage.from_blocks(dev, qt, 0, n, k, blocks), dev.storage_from_slice(x), dev.zeros(m * n)
+    lib, ctx = dev._lib, dev.ctx
+    call_it = lambda: abi.check(ctx, lib.cq_qmatmul(ctx, qt, 0, ACT_Q8_1, xd.ptr, m, k, k, qs.buf.ptr, n, yd.ptr, n), "matmul")  # noqa: E731
+    abi.check(ctx, lib.cq_reserve(ctx, room(m, k)), "reserve")
+    g = C.c_void_p()
+    abi.check(ctx, lib.cq_capture_begin(ctx), "begin")
+    try:
+        call_it()
+    finally:
+        abi.check(ctx, lib.cq_capture_end(ctx, C.byref(g)), "end")
+    abi.check(ctx, lib.cq_memset(ctx, yd.ptr, 0, 4 * m * n), "clear")
+    abi.check(ctx, lib.cq_graph_launch(ctx, g), "launch")
+    got = yd.data().reshape(m, n)
+    lib.cq_graph_destroy(ctx, g)
+    rows = np.unique(np.linspace(0, m - 1, 40).astype(int))
+    want = oc.qmatmul(qt, 0, x[rows], blocks, n, nthreads=8, q8_1=True).astype(np.float64)
+    assert (np.abs(got[rows] - want) <= (k // 32 + 4) * 2.0 ** -23 * terms(qt, 0, x[rows], blocks, n)).all()
+    dev.set_option("split_min_rows_q8_1", 0)
+    call_it()
+    integer = yd.data().reshape(m, n)
+    assert np.array_equal(got, integer) == (m == 1000)
+    del qs, xd, yd
+    dev.close()

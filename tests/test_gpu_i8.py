@@ -60,6 +60,22 @@ def test_f32_mode_batches_match_cpu_path(device, qt, order, m, n, k):
         assert rel_err(planes, want) < 1e-4
 
 
+@pytest.mark.parametrize("qt,order", QT_ORDERS)
+@pytest.mark.parametrize("m,n,k", [(33, 129, 512), (40, 2048, 4096), (128, 640, 768), (130, 257, 512), (300, 96, 256)])
+def test_q8_1_integer_dots_of_larger_batches(device, qt, order, m, n, k):
+    """Batches that products of f16 numbers serve unless they are captured with little scratch, or memory is short."""
+    w, x = make_case(7300 + m + n + k, n, k, m)
+    x[0, :32] = 0.0
+    x[m - 1, 32:64] *= 1e3
+    blocks = oc.quantize(qt, order, w)
+    device.set_option("split_min_rows_q8_1", 0)
+    try:
+        got = run(device, qt, order, x, blocks, n, 1)
+    finally:
+        device.set_option("split_min_rows_q8_1", 33)
+    assert rel_err(got, oc.qmatmul(qt, order, x, blocks, n, nthreads=16, q8_1=True)) < 2e-5
+
+
 def test_row_stride_of_y_and_repeatability(device):
     m, n, k = 6, 700, 1024
     w, x = make_case(7200, n, k, m)

@@ -37,15 +37,16 @@ __global__ void __launch_bounds__(256) gp_sum_kernel(const GpParams p) {
     const int r = (threadIdx.x % PER) * 4;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     const bool ends = (first * p.per_share) / p.nchunks != t;  // the first share had an earlier tile too: this one is its second slot
-    for (int c = first; c <= last; c += 8) {
-        float4 v[8];  // eight partial tiles in flight (one after the other, 19 of them took 8 us)
+    for (int c = first; c <= last; c += 4) {
+        // Four partial tiles in flight, and none twice.  (us of the call with one at a time / four / eight / eight whose loads past the
+        // last repeat it: f16 128 x 4096 x 4096 15.4 / 14.6 / 14.4 / 15.7, 128 x 11008 x 4096 22.6 / 22.2 / 22.8 / 22.7; f32 512 x 11008 x
+        // 4096 112.4 / 112.8 / 114.1 / 114.6; Q8_1 64 x 700 x 14336, 19 of them, 21.9 / 20.9 / 20.5 / 20.9.)
+        float4 v[4];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int share = min(c + u, last), slot = 2 * share + (share == first && ends ? 1 : 0);
-            v[u] = *reinterpret_cast<const float4 *>(p.part + ((int64_t)slot * NB + lc) * TILE + r);
-        }
+        for (int u = 0; u < 4; ++u)
+            if (c + u <= last) v[u] = *reinterpret_cast<const float4 *>(p.part + ((int64_t)(2 * (c + u) + (c + u == first && ends ? 1 : 0)) * NB + lc) * TILE + r);
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
+        for (int u = 0; u < 4; ++u)
             if (c + u <= last) acc.x += v[u].x, acc.y += v[u].y, acc.z += v[u].z, acc.w += v[u].w;
     }
     const int64_t j = (int64_t)group * TILE + r;

@@ -529,7 +529,9 @@ cq_status cq_qmatmul_host(cq_ctx *ctx, int qtype, int order, int actmode, const 
 // Page-locked blocks of the context for host buffers that are not page-locked themselves.  A copy between pageable memory and
 // the device goes through the driver's own block and waits for it twice: 17 of the 46 us that a 4096 x 4096 Q8_0 linear took on
 // one row.  Copying into such a block first and letting the copy engine, or the kernel's stores, work on that leaves one wait.
-// A megabyte a direction is kept; above that the driver's way costs little beside the transfer.
+// A megabyte a direction is kept.  QLinear.forward, us, the driver's copies / these blocks: 4096 x 4096 Q8_0, 1 row 54 / 42, 8 rows 75 /
+// 52..71, 16 rows 99 / 84..100, 32 rows 137 / 129..153, 64 rows (a megabyte) 231..270 / 223..240; 1024 x 1024, 1 row 43 / 27, 64 rows 91 /
+// 84; 11008 x 4096, 24 rows 181 / 180..184: the gain is gone where the copies themselves are the most of the call.
 static constexpr size_t kPinnedMax = size_t(1) << 20;
 
 static void *pinned_block(cq_ctx *ctx, void **block, size_t *have, size_t bytes) {
@@ -584,8 +586,9 @@ cq_status cq_qlinear_host(cq_ctx *ctx, int qtype, int order, int actmode, const 
     }
     CQ_CUDA(ctx, cudaMemcpyAsync(ctx->xfer_x, x_src, xb, cudaMemcpyHostToDevice, ctx->stream));
     // A result buffer in pinned host memory is written by the kernel itself (it is addressable from the device):
-    // no copy out, one submission less.  Only for the row-streaming kernels (m <= 8), which store every result
-    // once and coalesced, and only for small results: the stores cross PCIe.  (A bias may be added by a kernel of its own.)
+    // no copy out, one submission less.  Only up to eight rows, whose kernels (the row-streaming ones, and for three to eight rows of
+    // Q8_0 the integer GEMM) store every result once and coalesced, and only for small results: the stores cross PCIe.  (A bias may be
+    // added by a kernel of its own.)
     switch (memory_type(y_host, &mapped)) {
         case cudaMemoryTypeHost: y_mapped = mapped; break;
         case cudaMemoryTypeUnregistered:

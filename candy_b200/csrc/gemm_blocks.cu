@@ -14,10 +14,10 @@
 //
 // The int8 GEMM (gemm_i8_tmem.cu), which served these batches and still serves the small ones, has exact whole-number dots but
 // scales them by both operands' block scales in the epilogue, and an activation scale, the same in every lane, costs a warp
-// as much to fetch from shared memory as 32 different values.  us at n 11008 x k 4096, Q4_0 / Q8_0, before -> now: 64 rows 46 /
-// 39 -> 33 / 29.5, 100 rows 73 / 64 -> 39 / 38, 300 rows 217 / 188 -> 85 / 81.
+// as much to fetch from shared memory as 32 different values.  us at n 11008 x k 4096, calls back to back, Q4_0 / Q8_0, before ->
+// now: 64 rows 45 / 37 -> 32 / 30, 100 rows 73 / 63 -> 39 / 37, 300 rows 217 / 188 -> 85 / 81.
 // What bounds it: the way of a slot round the ring (MMAs, commit, poll, tensor-memory load, arrive, poll: about 1500 cycles),
-// three slots under way; the tensor pipe is half busy.  Measured on 512 rows of the same kernel in f32 arithmetic: sixteen
+// three slots under way; the tensor pipe is active in 57 / 48 % of the cycles, the issue slots in 55 % (100 rows, n 32000).  Measured on 512 rows of the same kernel in f32 arithmetic: sixteen
 // epilogue warps of 32 columns 107, eight of 64 103; sleeping polls 122; one issuing warp instead of two 111; on CTA pairs
 // (half the activation traffic, but barriers across the pair) 99 with sixteen warps.
 //

@@ -1,5 +1,5 @@
 """Prefill attention with two query tiles per CTA (cq_flash_attention, option fa_two_tiles = 2) against the CPU oracle, at the
-edges of its tiles (256 query rows, 128 keys), where rows change their reference, and on non-finite inputs against the kernel
+edges of its tiles (256 query rows, 128 keys), where later key tiles raise a maximum, and on non-finite inputs against the kernel
 with one tile.  Bars as for that kernel: the rounding of p to 16 bits (2^-9 in bf16, 2^-12 in f16) sets them."""
 import ctypes as C
 
@@ -66,7 +66,7 @@ def attend(device, q, k, v, scale, causal, bf16, option):
 @pytest.mark.parametrize("causal", [False, True])
 @pytest.mark.parametrize("growth", [3.0, 30.0, 300.0])
 def test_scores_that_grow_from_tile_to_tile(device, growth, causal, bf16):
-    """Every key tile's scores lie about `growth` above the last one's, in some rows only: new references and rescaled sums."""
+    """Every key tile's scores lie about `growth` above the last one's, in some rows only: new maxima and rescaled sums."""
     rng = np.random.default_rng(int(growth))
     sq, sk, d = 300, 600, 128
     q, k, v = (rng.standard_normal((1, s, h, d)).astype(np.float32) for s, h in ((sq, 4), (sk, 2), (sk, 2)))
